@@ -41,6 +41,36 @@ std::string& vfv_thread_error() {
 // ================================================================ GMRES driver
 namespace {
 
+// launch attributes: programmatic dependent launch after the previous kernel, stream priority
+inline void launch_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool pdl, int prio, bool use_prio) {
+    int na = 0;
+    if (pdl) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
+    if (use_prio) {
+        attr[na].id = cudaLaunchAttributePriority;
+        attr[na].val.priority = prio;
+        ++na;
+    }
+    cfg.attrs = na ? attr : nullptr;
+    cfg.numAttrs = na;
+}
+
+// k<<<grid, block, 0, s>>>(args...), with programmatic dependent launch after the stream's previous
+// kernel when pdl is set (k then waits with pdl_wait before it touches what that kernel writes)
+template <typename... KArgs, typename... Args>
+void launch_k(cudaStream_t s, void (*k)(KArgs...), int64_t grid, int block, bool pdl, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    launch_attrs(cfg, attr, pdl, 0, false);
+    cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+}
+
 // SpMV shapes: G lanes per row, each lane loading its first S strides of the row (indices and
 // values) before any gather. The autotuner picks one per pattern and precision; (G, 4) exists for
 // every G (the shape vfv_pattern_set_spmv_lanes selects).
@@ -53,32 +83,34 @@ constexpr int kSpmvShapes[][2] = {
 
 template <typename TV, typename TX, typename TY, typename TA>
 void launch_spmv(cudaStream_t s, int lanes, int strides, int64_t n, const int32_t* rp, const int32_t* ci, const TV* val, const TX* x,
-                 TY* y, const double* scale, const DevStatus* st) {
+                 TY* y, const double* scale, const DevStatus* st, bool pdl = false) {
     switch (lanes * 16 + strides) {
-#define VFV_SHAPE_CASE(G, S)                                                                                  \
-    case G * 16 + S:                                                                                          \
-        k_spmv<TV, TX, TY, TA, G, S><<<grid_for(n * G), kBlk, 0, s>>>(n, rp, ci, val, x, y, scale, st);         \
+#define VFV_SHAPE_CASE(G, S)                                                                                               \
+    case G * 16 + S:                                                                                                       \
+        launch_k(s, k_spmv<TV, TX, TY, TA, G, S>, grid_for(n * G), kBlk, pdl, n, rp, ci, val, x, y, scale, st);             \
         return;
         VFV_SPMV_SHAPES(VFV_SHAPE_CASE)
 #undef VFV_SHAPE_CASE
         default:
-            k_spmv<TV, TX, TY, TA, 4, 4><<<grid_for(n * 4), kBlk, 0, s>>>(n, rp, ci, val, x, y, scale, st);
+            launch_k(s, k_spmv<TV, TX, TY, TA, 4, 4>, grid_for(n * 4), kBlk, pdl, n, rp, ci, val, x, y, scale, st);
     }
 }
 
 // SpMV of a batched solve: the step's scale 1/beta_j looked up per row from its mesh
 template <typename TV, typename TX, typename TY, typename TA>
 void launch_spmv_seg(cudaStream_t s, int lanes, int strides, int64_t n, const int32_t* rp, const int32_t* ci, const TV* val, const TX* x,
-                     TY* y, const double* inv_beta, int stride, int j, const int64_t* mesh_row, int nm, const DevStatus* st) {
+                     TY* y, const double* inv_beta, int stride, int j, const int64_t* mesh_row, int nm, const DevStatus* st, bool pdl) {
     switch (lanes * 16 + strides) {
-#define VFV_SHAPE_CASE(G, S)                                                                                                         \
-    case G * 16 + S:                                                                                                                 \
-        k_spmv_seg<TV, TX, TY, TA, G, S><<<grid_for(n * G), kBlk, 0, s>>>(n, rp, ci, val, x, y, inv_beta, stride, j, mesh_row, nm, st); \
+#define VFV_SHAPE_CASE(G, S)                                                                                                          \
+    case G * 16 + S:                                                                                                                  \
+        launch_k(s, k_spmv_seg<TV, TX, TY, TA, G, S>, grid_for(n * G), kBlk, pdl, n, rp, ci, val, x, y, inv_beta, stride, j, mesh_row, \
+                 nm, st);                                                                                                             \
         return;
         VFV_SPMV_SHAPES(VFV_SHAPE_CASE)
 #undef VFV_SHAPE_CASE
         default:
-            k_spmv_seg<TV, TX, TY, TA, 4, 4><<<grid_for(n * 4), kBlk, 0, s>>>(n, rp, ci, val, x, y, inv_beta, stride, j, mesh_row, nm, st);
+            launch_k(s, k_spmv_seg<TV, TX, TY, TA, 4, 4>, grid_for(n * 4), kBlk, pdl, n, rp, ci, val, x, y, inv_beta, stride, j, mesh_row,
+                     nm, st);
     }
 }
 
@@ -344,23 +376,6 @@ int clone_ilu_struct(vfv_ctx* ctx, const IluStruct& F, int64_t nnz, IluStruct& S
     CK(S.bad.alloc(1));
     CK(cudaStreamSynchronize(s));
     return VFV_OK;
-}
-
-// launch attributes: programmatic dependent launch after the previous kernel, stream priority
-inline void launch_attrs(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool pdl, int prio, bool use_prio) {
-    int na = 0;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
-    if (use_prio) {
-        attr[na].id = cudaLaunchAttributePriority;
-        attr[na].val.priority = prio;
-        ++na;
-    }
-    cfg.attrs = na ? attr : nullptr;
-    cfg.numAttrs = na;
 }
 
 // numeric ILU(0) of the pattern's current values (double), cast to float when asked
@@ -808,6 +823,38 @@ cudaError_t ilu_apply_chain(cudaStream_t s, IluStruct& S, const T* lu, const T* 
                               reinterpret_cast<IluChainState*>(C.state.p), timeout_flag, st);
 }
 
+enum class VecShape { wide, mid, small };
+
+// fn(shape type) for a run-time shape
+template <typename F>
+void with_shape(VecShape v, F fn) {
+    if (v == VecShape::wide) fn(VecWide{});
+    else if (v == VecShape::mid) fn(VecMid{});
+    else fn(VecSmall{});
+}
+
+template <typename T>
+int64_t shape_rows(VecShape v) {
+    int64_t r = 0;
+    with_shape(v, [&](auto S) { r = vec_block_rows<T, decltype(S)>(); });
+    return r;
+}
+
+// The shape for vectors of `rows` rows (all meshes of a batch together), by the blocks of 256
+// 16-byte chunks that they make. Measured on one B200, whole solves, wide / mid / small: 16 blocks
+// (8,000 FP64 rows) 5.3 / 4.4 / 3.6 ms, 108 blocks 53 / 44 / 38 ms, 244 blocks 44.5 / 42.6 / 47.8 ms,
+// 512 blocks 34.9 / 33.8 / 40.3 ms, 977 blocks (10^6 float rows) 100.9 / 103 / 140 ms.
+template <typename T>
+VecShape vec_shape(int64_t rows) {
+    const int64_t blocks = (rows + shape_rows<T>(VecShape::wide) - 1) / shape_rows<T>(VecShape::wide);
+    return blocks >= 800 ? VecShape::wide : blocks >= 150 ? VecShape::mid : VecShape::small;
+}
+
+// Up to this many partials per vector the update kernels sum them themselves: two launches per
+// Arnoldi step less (8,000 rows: 3.57 against 3.65 ms per solve; 400 partials already cost more than
+// the launches they save, 130 against 118 ms at 131,072 rows).
+constexpr int kFoldMax = 128;
+
 constexpr int kStepsPerIf = 4;  // Arnoldi steps per IF node of a cycle graph
 
 // Sets the IF condition of the next group of Arnoldi steps of a cycle graph: run it unless the solve stopped.
@@ -818,7 +865,7 @@ struct Gmres : SolverBase {
     int64_t n = 0, ldv = 0;
     int m = 0, precond = 0, ilu_order = 0, engine = 0;
     int nblk = 0, mega_grid = 0, mega_chunk = 0;
-    int nblk_v = 0;       // blocks of the multi-vector kernels (vec_block_rows<T>() rows each)
+    VecShape shape = VecShape::wide;  // of the multi-vector kernels
     DBuf<T> V, z, z2, zc, valK;
     DBuf<unsigned> bar;
     DBuf<unsigned long long> trace;  // per-phase timestamps of the last cycle (VFV_TRACE_CYCLE=1)
@@ -856,7 +903,7 @@ struct Gmres : SolverBase {
     DBuf<int32_t> b_tile_mesh, b_mesh_tile, b_rtile_mesh, b_mesh_rtile;
     DBuf<double> b_part, b_rpart, b_hacc, b_coef, b_H, b_cs, b_sn, b_g, b_beta, b_inv_beta, b_y, b_tol;
     DBuf<MeshStat> b_ms;
-    DBuf<unsigned> b_counter;
+    DBuf<unsigned> b_counter, b_mesh_counter;
     BatchDev B{};
     std::vector<MeshStat> mesh_stat;  // per-mesh state after the last solve
     long long wait_polls = kDefaultWaitPolls;  // bounded device waits of this solve (vfv_gmres_opts::wait_limit)
@@ -879,8 +926,8 @@ struct Gmres : SolverBase {
         ortho = ortho_;
         sweep_half = sweep_half_ && sweeps > 0 && !std::is_same<T, double>::value;
         ldv = (n + 63) / 64 * 64;
-        nblk_v = (int)((n + vec_block_rows<T>() - 1) / vec_block_rows<T>());
-        nblk = nblk_v;  // partial dots per vector
+        shape = vec_shape<T>(n);
+        nblk = (int)((n + shape_rows<T>(shape) - 1) / shape_rows<T>(shape));  // partial dots per vector
         const int64_t res_blocks = (n * kSpG + kBlk - 1) / kBlk;
         CK(V.alloc((size_t)(m + 1) * ldv));
         CK(cudaMemset(V.p, 0, sizeof(T) * (size_t)(m + 1) * ldv));
@@ -924,7 +971,7 @@ struct Gmres : SolverBase {
                 }
             }
         }
-        CK(part.alloc(std::max<int64_t>((int64_t)kMaxBasis * std::max(nblk, mega_grid), res_blocks) + 16));
+        CK(part.alloc(std::max<int64_t>((int64_t)kMaxBasis * std::max(3 * nblk, mega_grid), res_blocks) + 16));
         CK(hacc.alloc(kMaxBasis));
         CK(coef.alloc(kMaxBasis));
         CK(H.alloc((size_t)m * (m + 1)));
@@ -948,6 +995,7 @@ struct Gmres : SolverBase {
         K.ldv = ldv;
         K.m = m;
         K.nblk = nblk;
+        K.fold = nblk <= kFoldMax;
         K.part = part.p;
         K.counter = counter.p;
         K.hacc = hacc.p;
@@ -991,20 +1039,22 @@ struct Gmres : SolverBase {
         return VFV_OK;
     }
 
-    // Tiles of the batched kernels from the mesh row ranges: vector tiles of vec_block_rows<T>() rows and
-    // residual tiles of kBlk / kSpG rows, each starting at its mesh's first row.
+    // Tiles of the batched kernels from the mesh row ranges, inside one mesh each: vector tiles that
+    // start on 16-byte boundaries but for a mesh's first, and residual tiles of kBlk / kSpG rows.
     int init_batch(vfv_ctx* ctx, const std::vector<int64_t>& rows) {
         nm = (int)rows.size() - 1;
         std::vector<int64_t> tr, rr;
         std::vector<int32_t> tm, mt(nm + 1), rm, mr(nm + 1);
-        const int64_t tv = vec_block_rows<T>(), tres = kBlk / kSpG;
+        const int64_t tv = shape_rows<T>(shape), tres = kBlk / kSpG;
+        int most = 0;  // vector tiles of a mesh
         for (int q = 0; q < nm; ++q) {
             mt[q] = (int32_t)tm.size();
             mr[q] = (int32_t)rm.size();
-            for (int64_t r = rows[q]; r < rows[q + 1]; r += tv) {
-                tr.push_back(r);
+            for (int64_t r = rows[q] / kVecRows<T> * kVecRows<T>; r < rows[q + 1]; r += tv) {
+                tr.push_back(std::max(r, rows[q]));
                 tm.push_back(q);
             }
+            most = std::max(most, (int)tm.size() - mt[q]);
             for (int64_t r = rows[q]; r < rows[q + 1]; r += tres) {
                 rr.push_back(r);
                 rm.push_back(q);
@@ -1023,8 +1073,8 @@ struct Gmres : SolverBase {
         CK(b_rtile_mesh.upload(rm.data(), rm.size(), s));
         CK(b_mesh_rtile.upload(mr.data(), mr.size(), s));
         const int ntile = (int)tm.size(), nrtile = (int)rm.size();
-        CK(b_part.alloc((size_t)kMaxBasis * ntile));
-        CK(b_rpart.alloc(nrtile));
+        CK(b_part.alloc((size_t)3 * kMaxBasis * ntile));
+        CK(b_rpart.alloc((size_t)2 * nrtile));
         CK(b_hacc.alloc((size_t)nm * kMaxBasis));
         CK(b_coef.alloc((size_t)nm * kMaxBasis));
         CK(b_H.alloc((size_t)nm * m * (m + 1)));
@@ -1038,6 +1088,9 @@ struct Gmres : SolverBase {
         CK(b_ms.alloc(nm));
         CK(b_counter.alloc(4));
         CK(cudaMemset(b_counter.p, 0, 4 * sizeof(unsigned)));
+        CK(b_mesh_counter.alloc(nm));
+        B.mesh_counter = b_mesh_counter.p;
+        B.fold = most <= kFoldMax;
         B.nm = nm;
         B.m = m;
         B.ldv = ldv;
@@ -1096,22 +1149,29 @@ struct Gmres : SolverBase {
     // unless the first pass's test asked for it; VFV_ORTHO_CGS: the first pass alone.
     void enqueue_ortho(cudaStream_t s, const T* win, T* w, int j) {
         const int nv = j + 1, fb = grid_for((int64_t)nv * 32), fb1 = grid_for((int64_t)(nv + 1) * 32);
-        if (ortho == VFV_ORTHO_CGS2) {
-            k_mdot<T><<<nblk, kBlk, 0, s>>>(K, V.p, win, nv, 0, 0);
-            k_dots_finish<true><<<fb, 256, 0, s>>>(K, nv, 0, 0);
-            k_update<T, false><<<nblk, kBlk, 0, s>>>(K, V.p, win, w, nv, j, 0, 0);
-            k_dots_finish<false><<<fb, 256, 0, s>>>(K, nv, 0, 0);
-            k_update<T, true><<<nblk, kBlk, 0, s>>>(K, V.p, w, w, nv, j, 0, 0);
-            return;
-        }
+        const bool cgs2 = ortho == VFV_ORTHO_CGS2, fold = K.fold != 0;
         const int dgks = ortho == VFV_ORTHO_DGKS ? 1 : 0;
-        k_mdot<T><<<nblk, kBlk, 0, s>>>(K, V.p, win, nv, dgks, 0);
-        k_dots_finish<true><<<dgks ? fb1 : fb, 256, 0, s>>>(K, nv, dgks, 0);
-        k_update<T, true><<<nblk, kBlk, 0, s>>>(K, V.p, win, w, nv, j, dgks, 0);
-        if (!dgks) return;
-        k_mdot<T><<<nblk, kBlk, 0, s>>>(K, V.p, w, nv, 0, 1);
-        k_dots_finish<false><<<fb, 256, 0, s>>>(K, nv, 0, 1);
-        k_update<T, true><<<nblk, kBlk, 0, s>>>(K, V.p, w, w, nv, j, 0, 1);
+        const T* basis = V.p;
+        // Programmatic dependent launch where the kernel or the one before it leaves most SMs free. A
+        // grid of one or two blocks per SM that starts among the last blocks of the one before lands
+        // unevenly on the SMs (FP64 solve of 125,000 rows 19.9 against 17.5 ms).
+        const bool pdl = shape == VecShape::small;
+        with_shape(shape, [&](auto sh) {
+            using S = decltype(sh);
+            launch_k(s, k_mdot<T, S>, nblk, kBlk, false, K, basis, win, nv, dgks, 0);
+            if (!fold) launch_k(s, k_dots_finish<true>, dgks ? fb1 : fb, 256, true, K, nv, dgks, 0);
+            if (cgs2) {
+                launch_k(s, k_update<T, S, false>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, 0, 0);
+                if (!fold) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 0);
+                launch_k(s, k_update<T, S, true>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 0);
+                return;
+            }
+            launch_k(s, k_update<T, S, true>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, dgks, 0);
+            if (!dgks) return;
+            launch_k(s, k_mdot<T, S>, nblk, kBlk, false, K, basis, w, nv, 0, 1);
+            if (!fold) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 1);
+            launch_k(s, k_update<T, S, true>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 1);
+        });
     }
 
     // phase timestamps of the last cycle, averaged over its steps (diagnostics, VFV_TRACE_CYCLE=1)
@@ -1234,25 +1294,30 @@ struct Gmres : SolverBase {
                 apply_ilu(s, uj, z.p, st.p);
                 in = z.p;
             }
-            launch_spmv_seg<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, w, b_inv_beta.p, m + 1, j, b_mesh_row.p, nm, st.p);
+            launch_spmv_seg<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, w, b_inv_beta.p, m + 1, j, b_mesh_row.p, nm, st.p, true);
             const int nv = j + 1, fb = grid_for((int64_t)nm * nv * 32);
-            k_bmdot<T><<<B.ntile, kBlk, 0, s>>>(B, V.p, w, nv);
-            k_bdots_finish<true><<<fb, 256, 0, s>>>(B, nv);
-            k_bupdate<T, false><<<B.ntile, kBlk, 0, s>>>(B, V.p, w, w, nv);
-            k_bdots_finish<false><<<fb, 256, 0, s>>>(B, nv);
-            k_bupdate<T, true><<<B.ntile, kBlk, 0, s>>>(B, V.p, w, w, nv);
-            k_bstep_finish<<<nm, kBlk, 0, s>>>(B, j);
+            const bool pdl = shape == VecShape::small;  // as in enqueue_ortho
+            with_shape(shape, [&](auto sh) {
+                using S = decltype(sh);
+                launch_k(s, k_bmdot<T, S>, B.ntile, kBlk, false, B, V.p, w, nv);
+                if (!B.fold) launch_k(s, k_bdots_finish<true>, fb, 256, true, B, nv);
+                launch_k(s, k_bupdate<T, S, false>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
+                if (!B.fold) launch_k(s, k_bdots_finish<false>, fb, 256, true, B, nv);
+                launch_k(s, k_bupdate<T, S, true>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
+            });
             return;
         }
         if (engine == VFV_ENGINE_OVERLAP) {
-            launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, Zb.p + (int64_t)j * ldv, abuf.p, inv_beta.p + j, st.p);
+            launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, Zb.p + (int64_t)j * ldv, abuf.p, inv_beta.p + j, st.p, true);
             cudaEventRecord(ev_fork, s);
             cudaStreamWaitEvent(s2, ev_fork, 0);
             apply_ilu(s2, abuf.p, qbuf.p, st.p, ilu_prio, true);
             cudaEventRecord(ev_join, s2);
             enqueue_ortho(s, abuf.p, w, j);
             cudaStreamWaitEvent(s, ev_join, 0);
-            k_zupdate<T><<<nblk_v, kBlk, 0, s>>>(K, Zb.p, qbuf.p, j + 1, j);
+            with_shape(shape, [&](auto sh) {
+                launch_k(s, k_zupdate<T, decltype(sh)>, nblk, kBlk, false, K, Zb.p, qbuf.p, j + 1, j);
+            });
             return;
         }
         const T* uj = V.p + (int64_t)j * ldv;
@@ -1261,10 +1326,10 @@ struct Gmres : SolverBase {
             apply_ilu(s, uj, z.p, st.p);
             in = z.p;
         } else if (precond == VFV_PRECOND_BJ4) {
-            k_bj4_apply<T><<<grid_for(n / 4), 256, 0, s>>>(n / 4, bj_vals(), uj, z.p, st.p);
+            launch_k(s, k_bj4_apply<T>, grid_for(n / 4), 256, true, n / 4, bj_vals(), uj, z.p, st.p);
             in = z.p;
         }
-        launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, w, inv_beta.p + j, st.p);
+        launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, w, inv_beta.p + j, st.p, true);
         enqueue_ortho(s, w, w, j);
     }
 
@@ -1273,7 +1338,7 @@ struct Gmres : SolverBase {
         const int sp_blocks = grid_for(n * G);
         const int vb = grid_for(n);
         if (nm > 0) {
-            k_bbacksolve<<<grid_for(nm, 128), 128, 0, s>>>(B);
+            k_bbacksolve<<<grid_for((int64_t)nm * 32, 128), 128, 0, s>>>(B);
             if (precond == VFV_PRECOND_ILU0) {
                 k_bcombine<T, 2><<<B.ntile, kBlk, 0, s>>>(B, V.p, x.p, nullptr, z.p);
                 apply_ilu(s, z.p, z.p, nullptr);
@@ -1283,8 +1348,8 @@ struct Gmres : SolverBase {
             } else {
                 k_bcombine<T, 0><<<B.ntile, kBlk, 0, s>>>(B, V.p, x.p, nullptr, nullptr);
             }
-            k_bresidual<T, G><<<B.nrtile, kBlk, 0, s>>>(B, p->rp.p, p->ci.p, p->val.p, x.p, b.p, V.p);
-            k_bresid_finish<<<nm, kBlk, 0, s>>>(B);
+            k_bresidual<T, G><<<B.nrtile, kBlk, 0, s>>>(B, p->rp.p, p->ci.p, p->val.p, x.p, b.p, V.p, 0);
+            k_bresid_finish<<<nm, kBlk, 0, s>>>(B, 0, 0.0);
             return;
         }
         k_backsolve<<<1, 32, 0, s>>>(K);
@@ -1450,11 +1515,10 @@ struct Gmres : SolverBase {
             const double hs[2] = {0.0, mixed ? std::max(0.0, o.inner_rtol) : 0.0};
             CK(cudaMemcpyAsync(scal.p, hs, 2 * sizeof(double), cudaMemcpyHostToDevice, s));
             CK(cudaMemsetAsync(st.p, 0, sizeof(DevStatus), s));
-            k_bnorm<<<nm, kBlk, 0, s>>>(B, b.p, o.tol);
+            k_bresidual<T, G><<<B.nrtile, kBlk, 0, s>>>(B, p->rp.p, p->ci.p, p->val.p, x.p, b.p, V.p, 1);
+            k_bresid_finish<<<nm, kBlk, 0, s>>>(B, 1, o.tol);
             k_bzero_x<<<grid_for(n), 256, 0, s>>>(B, x.p);
-            k_bresidual<T, G><<<B.nrtile, kBlk, 0, s>>>(B, p->rp.p, p->ci.p, p->val.p, x.p, b.p, V.p);
-            k_bresid_finish<<<nm, kBlk, 0, s>>>(B);
-            ctx->launches += 4;
+            ctx->launches += 3;
             if (info) info->levels = ilu ? ilu->nlev : 0;
         } else {
             // ||b|| and the absolute tolerance

@@ -30,6 +30,13 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
     return s;
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start its prologue / wait until
+// the previous kernel has finished and its writes are visible (both do nothing in a kernel launched
+// without the attribute). A kernel in such a chain waits on every path, early exits included: the
+// kernel after it waits for this one alone.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename T>
 __device__ __forceinline__ T ldg_stream(const T* p) { return __ldcs(p); }
 

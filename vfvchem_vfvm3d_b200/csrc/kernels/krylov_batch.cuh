@@ -8,10 +8,10 @@
 // `done` flag. A mesh that has converged (or finished its m steps of the cycle) is masked out of the
 // orthogonalisation kernels; the cycle ends once every mesh is done.
 //
-// Bitwise equality with a mesh solved alone: the vector kernels work on tiles of vec_block_rows<T>()
-// rows that start at each mesh's first row (the single-system kernels' blocks, shifted), the residual on
-// tiles of kBlk / kSpG rows, and every per-mesh sum uses the single-system kernels' reduction order
-// over the mesh's own tiles, so a mesh's iterates do not depend on the rest of the batch.
+// A mesh's iterates do not depend on the rest of the batch: the vector kernels work on tiles that lie
+// inside one mesh (the single-system kernels' tiles; the first one of a mesh that starts off a
+// 16-byte boundary is shorter by the offset, so that all others are aligned), the residual on tiles
+// of kBlk / kSpG rows, and every per-mesh sum runs over the mesh's own tiles in a fixed order.
 #pragma once
 #include "krylov.cuh"
 
@@ -34,15 +34,16 @@ struct BatchDev {
     int nm, m;
     int64_t ldv;
     const int64_t* mesh_row;   // [nm+1] first row of each mesh
-    const int64_t* tile_row;   // [ntile+1] vector tiles (vec_block_rows<T>() rows, inside one mesh)
+    const int64_t* tile_row;   // [ntile+1] vector tiles (at most vec_block_rows rows, inside one mesh)
     const int32_t* tile_mesh;  // [ntile]
     const int32_t* mesh_tile;  // [nm+1]
     const int64_t* rtile_row;  // [nrtile+1] residual tiles (kBlk / kSpG rows, inside one mesh)
     const int32_t* rtile_mesh; // [nrtile]
     const int32_t* mesh_rtile; // [nm+1]
     int ntile, nrtile;
-    double* part;              // [kMaxBasis][ntile] per-tile partial dots
-    double* rpart;             // [nrtile] per-tile partial residual norms
+    int fold;                  // the update kernels sum the mesh's partial dots themselves (no k_bdots_finish)
+    double* part;              // [3][kMaxBasis][ntile] per-tile partial dots: first pass, second pass, ||w||^2
+    double* rpart;             // [2][nrtile] per-tile partial norms of the residual and of b
     double* hacc;              // [nm][kMaxBasis]
     double* coef;              // [nm][kMaxBasis]
     double* H;                 // [nm][m][m+1] column-major per mesh
@@ -54,7 +55,8 @@ struct BatchDev {
     double* y;                 // [nm][m]
     double* tol_abs;           // [nm] tol * ||b_mesh||
     MeshStat* ms;              // [nm]
-    unsigned* counter;         // [4] arrival / done counters of the per-mesh finish kernels
+    unsigned* counter;         // [0] arrivals, [1] done and [2] converged meshes at a cycle's start, [3] active meshes
+    unsigned* mesh_counter;    // [nm] tiles of the mesh that have arrived in k_bupdate<FINAL>
     DevStatus* st;             // global: done once every mesh is done
     const double* scal;        // [1]: mixed precision, a mesh's cycle also ends at resid_est <= scal[1] * beta0
 };
@@ -72,39 +74,25 @@ __device__ __forceinline__ int mesh_of_row(const int64_t* __restrict__ mesh_row,
 // y = (A x) * inv_beta[mesh(row)][j]: the single-system SpMV with the step's scale looked up per row.
 template <typename TV, typename TX, typename TY, typename TA, int G, int S = 4>
 __global__ void __launch_bounds__(kBlk) k_spmv_seg(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                                  const TV* __restrict__ val, const TX* __restrict__ x, TY* __restrict__ y,
-                                                  const double* __restrict__ inv_beta, int stride, int j,
-                                                  const int64_t* __restrict__ mesh_row, int nm, const DevStatus* __restrict__ st) {
-    if (st->done) return;
+                                                  const TV* __restrict__ val, const TX* x, TY* y, const double* inv_beta, int stride, int j,
+                                                  const int64_t* __restrict__ mesh_row, int nm, const DevStatus* st) {
     const int lane = threadIdx.x & (G - 1);
     const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const bool skip = st->done;  // set once and for all within a cycle: such a launch loads no rows
+    RowFrag<TV, S> f;
+    int mesh = 0;
+    if (row < n) {
+        row_load<TV, G, S>(f, rp, ci, val, row, lane, skip);
+        mesh = mesh_of_row(mesh_row, nm, row);
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    if (skip || st->done) return;
     TA s = TA(0);
-    if (row < n) s = row_dot<TV, TX, TA, G, S>(rp, ci, val, x, row, lane);
+    if (row < n) s = row_gather<TV, TX, TA, G, S>(f, ci, val, x, lane);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, G);
-    if (lane == 0 && row < n) {
-        const double sc = inv_beta[(int64_t)mesh_of_row(mesh_row, nm, row) * stride + j];
-        y[row] = (TY)((double)s * sc);
-    }
-}
-
-// ||b_mesh||^2 and the mesh tolerance; one CTA per mesh.
-__global__ void __launch_bounds__(kBlk) k_bnorm(BatchDev B, const double* __restrict__ b, double tol) {
-    __shared__ double red[kBlk / 32];
-    const int m = blockIdx.x;
-    const int64_t r0 = B.mesh_row[m], r1 = B.mesh_row[m + 1];
-    double s = 0.0;
-    for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) s += b[i] * b[i];
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) {
-        const double bn = sqrt(s);
-        MeshStat& M = B.ms[m];
-        M = MeshStat{};
-        M.bnorm = bn;
-        M.zero_rhs = bn == 0.0 ? 1 : 0;
-        M.nonfinite = isfinite(bn) ? 0 : 1;
-        B.tol_abs[m] = tol * bn;
-    }
+    if (lane == 0 && row < n) y[row] = (TY)((double)s * inv_beta[(int64_t)mesh * stride + j]);
 }
 
 // x = 0 on meshes whose right-hand side is zero (their solution)
@@ -115,15 +103,16 @@ __global__ void k_bzero_x(BatchDev B, double* __restrict__ x) {
     if (B.ms[mesh_of_row(B.mesh_row, B.nm, row)].zero_rhs) x[row] = 0.0;
 }
 
-// r = b - A x per residual tile (FP64), u0 = r, per-tile ||r||^2 (k_residual's arithmetic).
+// r = b - A x per residual tile (FP64), u0 = r, per-tile ||r||^2 (k_residual's arithmetic). first: the
+// start of a solve, every mesh takes part and the tile's ||b||^2 is summed as well.
 template <typename T, int G>
 __global__ void __launch_bounds__(kBlk) k_bresidual(BatchDev B, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                                    const double* __restrict__ val, const double* __restrict__ x,
-                                                   const double* __restrict__ b, T* __restrict__ u0) {
+                                                   const double* __restrict__ b, T* __restrict__ u0, int first) {
     __shared__ double red[kBlk / 32];
     const int t = blockIdx.x;
     const MeshStat& M = B.ms[B.rtile_mesh[t]];
-    if (M.converged || M.zero_rhs) return;  // frozen mesh: no residual, no partial (its finish skips it)
+    if (!first && (M.converged || M.zero_rhs)) return;  // frozen mesh: no residual, no partial (its finish skips it)
     const int lane = threadIdx.x & (G - 1);
     const int64_t row = B.rtile_row[t] + threadIdx.x / G;
     const bool in = row < B.rtile_row[t + 1];
@@ -131,56 +120,70 @@ __global__ void __launch_bounds__(kBlk) k_bresidual(BatchDev B, const int32_t* _
     if (in) s = row_dot<double, double, double, G>(rp, ci, val, x, row, lane);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, G);
-    double r2 = 0.0;
+    double r2 = 0.0, b2 = 0.0;
     if (lane == 0 && in) {
-        const double r = b[row] - s;
+        const double bv = b[row], r = bv - s;
         u0[row] = (T)r;
         r2 = r * r;
+        b2 = bv * bv;
     }
-    const double bs = block_sum(r2, red);
-    if (threadIdx.x == 0) B.rpart[t] = bs;
+    const double rs = block_sum(r2, red);
+    if (threadIdx.x == 0) B.rpart[t] = rs;
+    if (first) {
+        const double bs = block_sum(b2, red);
+        if (threadIdx.x == 0) B.rpart[B.nrtile + t] = bs;
+    }
 }
 
-// Arrival of one finish CTA: counts `done` meshes; the last arrival publishes the global flags and
-// resets the counters. counter[0] arrivals, [1] done meshes, [2] converged meshes, [3] active meshes.
-__device__ __forceinline__ void batch_arrive(const BatchDev& B, bool done, bool conv, bool active, bool cycle_start) {
+// Arrival of one mesh's k_bresid_finish CTA: counts the done and converged meshes; the last arrival
+// publishes the global flags and resets the counters.
+__device__ __forceinline__ void batch_arrive(const BatchDev& B, bool done, bool conv) {
     __threadfence();
     if (done) atomicAdd(B.counter + 1, 1u);
     if (conv) atomicAdd(B.counter + 2, 1u);
-    if (active) atomicAdd(B.counter + 3, 1u);
     __threadfence();
     const unsigned t = atomicAdd(B.counter, 1u);
     if (t == (unsigned)B.nm - 1) {
         __threadfence();
-        const unsigned nd = atomicAdd(B.counter + 1, 0u), nc = atomicAdd(B.counter + 2, 0u), na = atomicAdd(B.counter + 3, 0u);
+        const unsigned nd = atomicAdd(B.counter + 1, 0u), nc = atomicAdd(B.counter + 2, 0u);
         DevStatus* st = B.st;
-        if (cycle_start) {
-            st->steps = 0;
-            st->converged = nc == (unsigned)B.nm ? 1 : 0;
-        } else if (na > 0) {
-            st->steps += 1;
-            st->total_steps += 1;
-        }
+        st->total_steps += st->steps;  // the cycle's steps: its longest mesh's (k_bbacksolve)
+        st->steps = 0;
+        st->converged = nc == (unsigned)B.nm ? 1 : 0;
         st->done = nd == (unsigned)B.nm ? 1 : 0;
-        B.counter[0] = B.counter[1] = B.counter[2] = B.counter[3] = 0u;
+        B.counter[0] = B.counter[1] = B.counter[2] = 0u;
+        B.counter[3] = (unsigned)B.nm - nd;
         __threadfence();
     }
 }
 
-// Start of a cycle per mesh (k_residual's last block): beta0, g, the convergence test. One CTA per mesh.
-__global__ void __launch_bounds__(kBlk) k_bresid_finish(BatchDev B) {
+// Start of a cycle per mesh (k_residual's last block): beta0, g, the convergence test. One CTA per
+// mesh. first (a solve's start): also ||b_mesh||, the mesh's tolerance and its fresh state; a mesh
+// with b = 0 is done (k_bzero_x sets its x).
+__global__ void __launch_bounds__(kBlk) k_bresid_finish(BatchDev B, int first, double tol) {
     __shared__ double red[kBlk / 32];
     const int m = blockIdx.x;
     MeshStat* M = B.ms + m;
-    const bool frozen = M->converged || M->zero_rhs;
-    double tot = 0.0;
-    if (!frozen) {
-        const int t0 = B.mesh_rtile[m], nt = B.mesh_rtile[m + 1] - t0;
-        tot = reduce_partials(B.rpart + t0, nt, red);
+    const int t0 = B.mesh_rtile[m], nt = B.mesh_rtile[m + 1] - t0;
+    const bool frozen = !first && (M->converged || M->zero_rhs);
+    double tot = 0.0, bb = 0.0;
+    if (!frozen) tot = reduce_partials(B.rpart + t0, nt, red);
+    if (first) {
+        __syncthreads();
+        bb = reduce_partials(B.rpart + B.nrtile + t0, nt, red);
     }
     if (threadIdx.x != 0) return;
-    bool conv = frozen;
-    if (!frozen) {
+    if (first) {
+        const double bn = sqrt(bb);
+        *M = MeshStat{};
+        M->bnorm = bn;
+        M->zero_rhs = bn == 0.0 ? 1 : 0;
+        M->nonfinite = isfinite(bn) ? 0 : 1;
+        B.tol_abs[m] = tol * bn;
+        B.mesh_counter[m] = 0u;
+    }
+    bool conv = frozen || M->zero_rhs;
+    if (!conv) {
         const int m1 = B.m + 1;
         const double beta0 = sqrt(tot);
         B.beta[(int64_t)m * m1] = beta0;
@@ -200,26 +203,35 @@ __global__ void __launch_bounds__(kBlk) k_bresid_finish(BatchDev B) {
         M->steps = 0;
         M->converged = 1;
     }
-    batch_arrive(B, M->done != 0, conv, false, true);
+    batch_arrive(B, M->done != 0, conv);
+}
+
+// The tile of block t: chunks on 16-byte boundaries, rows outside the tile masked.
+template <typename T, class S>
+__device__ __forceinline__ VecTile<T, S> batch_tile(const BatchDev& B, int t) {
+    const int32_t beg = (int32_t)B.tile_row[t];
+    return VecTile<T, S>(beg & ~(kVecRows<T> - 1), beg, (int32_t)B.tile_row[t + 1]);
 }
 
 // First CGS pass: per-tile partial dots of the mesh's basis with w (k_mdot per tile).
-template <typename T>
-__global__ void __launch_bounds__(kBlk, kVecMinBlocks) k_bmdot(BatchDev B, const T* __restrict__ V, const T* __restrict__ w, int nvec) {
+template <typename T, class S>
+__global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bmdot(BatchDev B, const T* V, const T* w, int nvec) {
+    pdl_wait();
+    pdl_launch_dependents();
     if (B.st->done) return;
     const int t = blockIdx.x;
     if (B.ms[B.tile_mesh[t]].done) return;
     __shared__ double red[kMaxBasis][kBlk / 32];
-    constexpr int R = kVecRows<T>;
-    const int nw = blockDim.x >> 5;
-    const int64_t row0 = B.tile_row[t] + (int64_t)R * threadIdx.x, end = B.tile_row[t + 1];
+    constexpr int R = kVecRows<T>, NW = VecTile<T, S>::kWarps;
+    const VecTile<T, S> q = batch_tile<T, S>(B, t);
     T wt[R];
-    load_chunk(w, row0, end, wt);
-    group_dots(V, B.ldv, row0, end, wt, nvec, red);
+    load_chunk(w + q.row0, q.lo, q.hi, wt);
+    group_dots<T, S>(V, B.ldv, q, wt, nvec, red);
     __syncthreads();
     for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
         double s = 0.0;
-        for (int q = 0; q < nw; ++q) s += red[i][q];
+#pragma unroll
+        for (int v = 0; v < NW; ++v) s += red[i][v];
         B.part[(int64_t)i * B.ntile + t] = s;
     }
 }
@@ -227,6 +239,8 @@ __global__ void __launch_bounds__(kBlk, kVecMinBlocks) k_bmdot(BatchDev B, const
 // Per-mesh cross-tile sums (k_dots_finish over the mesh's tiles): one warp per (mesh, vector).
 template <bool FIRST>
 __global__ void __launch_bounds__(256) k_bdots_finish(BatchDev B, int nvec) {
+    pdl_wait();
+    pdl_launch_dependents();
     if (B.st->done) return;
     const int lane = threadIdx.x & 31;
     const int64_t wgl = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -234,7 +248,7 @@ __global__ void __launch_bounds__(256) k_bdots_finish(BatchDev B, int nvec) {
     const int m = (int)(wgl / nvec), c = (int)(wgl % nvec);
     if (B.ms[m].done) return;
     const int t0 = B.mesh_tile[m], nt = B.mesh_tile[m + 1] - t0;
-    const double* p = B.part + (int64_t)c * B.ntile + t0;
+    const double* p = B.part + (int64_t)((FIRST ? 0 : kMaxBasis) + c) * B.ntile + t0;
     constexpr int kB = 16;
     double s = 0.0;
     for (int q0 = 0; q0 < nt; q0 += 32 * kB) {
@@ -261,123 +275,114 @@ __global__ void __launch_bounds__(256) k_bdots_finish(BatchDev B, int nvec) {
 }
 
 // w <- win - sum_i coef_i u_i per tile; FINAL == false: second-pass partial dots; FINAL == true:
-// per-tile ||w||^2 (k_update's arithmetic).
-template <typename T, bool FINAL>
-__global__ void __launch_bounds__(kBlk, kVecMinBlocks) k_bupdate(BatchDev B, const T* __restrict__ V, const T* win, T* w, int nvec) {
+// per-tile ||w||^2, and the mesh's last tile to arrive completes its Arnoldi step j: Hessenberg
+// column, Givens rotation, stopping test (k_update's arithmetic). The last mesh to stop sets the
+// global done flag.
+template <typename T, class S, bool FINAL>
+__global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, const T* V, const T* win, T* w, int nvec, int j) {
+    pdl_wait();
+    pdl_launch_dependents();
     if (B.st->done) return;
     const int t = blockIdx.x;
     const int m = B.tile_mesh[t];
-    if (B.ms[m].done) return;
-    __shared__ double red[kMaxBasis][kBlk / 32];
-    __shared__ double red2[kBlk / 32];
+    MeshStat* M = B.ms + m;
+    if (M->done) return;
+    constexpr int R = kVecRows<T>, NW = VecTile<T, S>::kWarps;
+    __shared__ double red[FINAL ? 1 : kMaxBasis][kBlk / 32];
     __shared__ double s_coef[kMaxBasis];
-    constexpr int R = kVecRows<T>;
-    const int nw = blockDim.x >> 5;
-    for (int i = threadIdx.x; i < nvec; i += blockDim.x) s_coef[i] = B.coef[(int64_t)m * kMaxBasis + i];
+    __shared__ double s_acc[S::kVS > 1 ? kBlk * R : 1];
+    __shared__ ColumnSmem s_col;
+    const int m1 = B.m + 1;
+    const int t0 = B.mesh_tile[m], nt = B.mesh_tile[m + 1] - t0;
+    double* hacc = B.hacc + (int64_t)m * kMaxBasis;
+    double* cs = B.cs + (int64_t)m * B.m;
+    double* sn = B.sn + (int64_t)m * B.m;
+    const double* inv_beta = B.inv_beta + (int64_t)m * m1;
+    if (B.fold) {
+        sum_columns(B.part + (FINAL ? (int64_t)kMaxBasis * B.ntile : 0) + t0, B.ntile, nt, nvec, [&](int c, double s) {
+            const double ib = inv_beta[c], hc = s * ib;
+            s_coef[c] = hc * ib;
+            s_col.h[c] = FINAL ? hacc[c] + hc : hc;
+            if (!FINAL && t == t0) hacc[c] = hc;
+        });
+    } else {
+        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+            s_coef[i] = B.coef[(int64_t)m * kMaxBasis + i];
+            if (FINAL) s_col.h[i] = hacc[i];
+        }
+    }
+    if (FINAL)
+        for (int i = threadIdx.x; i < j; i += blockDim.x) {
+            s_col.cs[i] = cs[i];
+            s_col.sn[i] = sn[i];
+        }
     __syncthreads();
-    const int64_t row0 = B.tile_row[t] + (int64_t)R * threadIdx.x, end = B.tile_row[t + 1];
+    const VecTile<T, S> q = batch_tile<T, S>(B, t);
     double acc[R];
-    group_combine(V, B.ldv, row0, end, s_coef, nvec, acc);
+    group_combine<T, S>(V, B.ldv, q, s_coef, nvec, acc, s_acc);
     T wt[R];
-    load_chunk(win, row0, end, wt);
+    load_chunk(win + q.row0, q.lo, q.hi, wt);
 #pragma unroll
-    for (int r = 0; r < R; ++r) wt[r] = (T)((double)wt[r] - acc[r]);  // rows past the end: 0 - 0
-    store_chunk(w, row0, end, wt);
+    for (int r = 0; r < R; ++r) wt[r] = (T)((double)wt[r] - acc[r]);  // rows outside the tile: 0 - 0
+    if (S::kVS > 1) __syncthreads();  // every group has read win before group 0 overwrites it (win may be w)
+    if (q.g() == 0) store_chunk(w + q.row0, q.lo, q.hi, wt);
     if (!FINAL) {
-        group_dots(V, B.ldv, row0, end, wt, nvec, red);
+        group_dots<T, S>(V, B.ldv, q, wt, nvec, red);
         __syncthreads();
+        double* part = B.part + (int64_t)kMaxBasis * B.ntile;
         for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
             double s = 0.0;
-            for (int q = 0; q < nw; ++q) s += red[i][q];
-            B.part[(int64_t)i * B.ntile + t] = s;
+#pragma unroll
+            for (int v = 0; v < NW; ++v) s += red[i][v];
+            part[(int64_t)i * B.ntile + t] = s;
         }
     } else {
         double s = 0.0;
+        if (q.g() == 0) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) s += (double)wt[r] * (double)wt[r];
-        s = block_sum(s, red2);
-        if (threadIdx.x == 0) B.part[t] = s;
-    }
-}
-
-// End of Arnoldi step j per mesh (k_update<true>'s last block): norm, Hessenberg column, Givens
-// rotation, convergence test. One CTA per mesh.
-__global__ void __launch_bounds__(kBlk) k_bstep_finish(BatchDev B, int j) {
-    if (B.st->done) return;
-    __shared__ double red[kBlk / 32];
-    const int m = blockIdx.x;
-    MeshStat* M = B.ms + m;
-    const bool active = !M->done;
-    double tot = 0.0;
-    if (active) {
-        const int t0 = B.mesh_tile[m], nt = B.mesh_tile[m + 1] - t0;
-        tot = reduce_partials(B.part + t0, nt, red);
-    }
-    if (threadIdx.x != 0) return;
-    if (active) {
-        const int m1 = B.m + 1;
-        double* col = B.H + ((int64_t)m * B.m + j) * m1;
-        const double* hacc = B.hacc + (int64_t)m * kMaxBasis;
-        double* cs = B.cs + (int64_t)m * B.m;
-        double* sn = B.sn + (int64_t)m * B.m;
+            for (int r = 0; r < R; ++r) s += (double)wt[r] * (double)wt[r];
+        }
+        s = block_sum(s, red[0]);
+        double* part = B.part + (int64_t)2 * kMaxBasis * B.ntile;
+        __shared__ bool s_last;
+        if (threadIdx.x == 0) {
+            publish_partial(part + t, s);
+            s_last = atomicAdd(B.mesh_counter + m, 1u) == (unsigned)nt - 1;
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        const double tot = reduce_partials(part + t0, nt, red[0]);
         double* g = B.g + (int64_t)m * m1;
-        const double bnext = sqrt(tot);
-        for (int i = 0; i <= j; ++i) col[i] = hacc[i];
-        col[j + 1] = bnext;
-        B.beta[(int64_t)m * m1 + j + 1] = bnext;
-        B.inv_beta[(int64_t)m * m1 + j + 1] = 1.0 / bnext;
-        for (int i = 0; i < j; ++i) {
-            const double a = col[i], bb = col[i + 1];
-            col[i] = cs[i] * a + sn[i] * bb;
-            col[i + 1] = -sn[i] * a + cs[i] * bb;
-        }
-        const double a = col[j], bb = col[j + 1];
-        const double rr = hypot(a, bb);
-        double c = 1.0, sgn = 0.0;
-        if (rr > 0.0) {
-            c = a / rr;
-            sgn = bb / rr;
-        }
-        cs[j] = c;
-        sn[j] = sgn;
-        col[j] = rr;
-        col[j + 1] = 0.0;
-        const double gj = g[j];
-        g[j] = c * gj;
-        g[j + 1] = -sgn * gj;
-        const double est = fabs(g[j + 1]);
+        const ColumnDst D{B.H + ((int64_t)m * B.m + j) * m1, cs, sn, g, B.beta + (int64_t)m * m1, B.inv_beta + (int64_t)m * m1};
+        const ColumnEnd c = arnoldi_column(D, s_col, j, tot);
+        if (threadIdx.x != 0) return;
+        B.mesh_counter[m] = 0u;
         M->steps = j + 1;
         M->total_steps += 1;
-        M->resid_est = est;
-        const bool fin = isfinite(est) && isfinite(bnext) && isfinite(rr);
+        M->resid_est = c.est;
+        const bool fin = isfinite(c.est) && isfinite(c.bnext) && isfinite(c.rr);
         if (!fin) {
             M->nonfinite = 1;
             B.st->nonfinite = 1;
         }
         const double floor_abs = B.scal[1] * M->beta0;
-        const bool stop = !fin || rr == 0.0 || bnext == 0.0 || est <= B.tol_abs[m] || est <= floor_abs || j + 1 >= B.m;
-        if (stop) M->done = 1;
+        if (!fin || c.rr == 0.0 || c.bnext == 0.0 || c.est <= B.tol_abs[m] || c.est <= floor_abs || j + 1 >= B.m) {
+            M->done = 1;
+            __threadfence();
+            if (atomicSub(B.counter + 3, 1u) == 1u) B.st->done = 1;
+        }
     }
-    batch_arrive(B, M->done != 0, false, active, false);
 }
 
-// Back substitution per mesh (k_backsolve), one thread per mesh.
-__global__ void k_bbacksolve(BatchDev B) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+// Back substitution per mesh (k_backsolve), one warp per mesh; the cycle's step count is its longest mesh's.
+__global__ void __launch_bounds__(128) k_bbacksolve(BatchDev B) {
+    const int m = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (m >= B.nm) return;
     const int k = B.ms[m].converged ? 0 : B.ms[m].steps;
     const int m1 = B.m + 1;
-    const double* H = B.H + (int64_t)m * B.m * m1;
-    const double* g = B.g + (int64_t)m * m1;
-    const double* ib = B.inv_beta + (int64_t)m * m1;
-    double* y = B.y + (int64_t)m * B.m;
-    for (int i = k - 1; i >= 0; --i) {
-        double s = g[i];
-        for (int q = i + 1; q < k; ++q) s -= H[(int64_t)q * m1 + i] * y[q];
-        y[i] = s / H[(int64_t)i * m1 + i];
-    }
-    for (int i = 0; i < k; ++i) y[i] *= ib[i];
-    for (int i = k; i < B.m; ++i) y[i] = 0.0;
+    if ((threadIdx.x & 31) == 0 && k > 0) atomicMax(&B.st->steps, k);
+    back_substitute(B.H + (int64_t)m * B.m * m1, m1, k, B.m, B.g + (int64_t)m * m1, B.inv_beta + (int64_t)m * m1, B.y + (int64_t)m * B.m);
 }
 
 // z = sum_i y_i u_i over the mesh's steps of this cycle (k_combine per row). MODE 0: x += z;
