@@ -295,7 +295,7 @@ int vfv_transport_adjoint_D(vfv_ctx* ctx, vfv_transport* t, const double* c0, in
  * (OpVecBndDirichlet + OpSclBndDivergence + OpSclBndPressureStabilizer per boundary) and whose
  * pressure is fixed at one vertex (OpSclDomPressureReference, opscl_dom_pref.rs:40-64), with the
  * Rhie-Chow flow data of flow_helper::update_flow (src/operator/core/flow_helper.rs:3-179). Pattern:
- * bit-exact to the reference's triplet build; values: the row's triplets summed in push order. */
+ * bit-exact to the reference's triplet build; values: the row's triplets, summed in a fixed order. */
 typedef struct vfv_flow vfv_flow;
 
 /* Symbolic setup only, on the host (no device): nnz and triplet count of the system, and its CSR

@@ -19,11 +19,14 @@ struct vfv_flow {
     vfv_ctx* ctx = nullptr;
     int64_t n = 0, n_pts = 0, n_dir = 0, n_bsub = 0, n_gc = 0, ntrip = 0, pref_vid = 0;
     double pref = 0.0, rho_max = 0.0;
-    DBuf<int32_t> np, ni, bp, bj, bk, gcp, gcv, div_off, pst_off, sub_off, slot_loc;
+    DBuf<int32_t> np, ni, bp, bj, bk, gcp, gcv, dloc, qlen, qself, rself;
+    DBuf<unsigned char> qring, rring, qnb, rgc, rnb, qsub;  // places in the p rows (NsLayout)
     DBuf<double> dist, area, norm, skew, gw, cvol, cskew, barea, bnorm, bw, gcc;
-    DBuf<double> den, visc, fce, bc_vel, gfix, gvel, rc, mom, flux, tv, b, x, xu;
+    DBuf<double> den, visc, fce, bc_vel, gfix, gvel, rc, mom, flux, gsum, b, x, xu;
     DBuf<double> xo, rpart;  // previous Picard state and the partials of its scaled change (device)
-    DBuf<int64_t> trip_ptr, slot_ptr;
+    DBuf<int64_t> qoff, roff;
+    bool wide = false;
+    int max_len = 0;
     vfv_pattern* pat = nullptr;
     ~vfv_flow() {
         if (pat) vfv_pattern_destroy(pat);
@@ -67,15 +70,23 @@ struct vfv_flow {
         D.rc = rc.p;
         D.mom = mom.p;
         D.flux = flux.p;
-        D.trip_ptr = trip_ptr.p;
-        D.div_off = div_off.p;
-        D.pst_off = pst_off.p;
-        D.sub_off = sub_off.p;
-        D.tv = tv.p;
+        D.dloc = dloc.p;
+        D.gsum = gsum.p;
+        D.qlen = qlen.p;
+        D.qself = qself.p;
+        D.rself = rself.p;
+        D.qoff = qoff.p;
+        D.roff = roff.p;
+        D.qring = qring.p;
+        D.rring = rring.p;
+        D.qnb = qnb.p;
+        D.rgc = rgc.p;
+        D.rnb = rnb.p;
+        D.qsub = qsub.p;
+        D.wide = wide;
+        D.max_len = max_len;
         D.b = b.p;
         D.rp = pat->rp.p;
-        D.slot_ptr = slot_ptr.p;
-        D.slot_loc = slot_loc.p;
         D.val = pat->val.p;
         return D;
     }
@@ -209,7 +220,7 @@ int flow_assemble(vfv_ctx* ctx, vfv_flow* f, const double* xs) {
     const double* fv[3] = {xs, xs + n, xs + 2 * n};
     launch_grad(s, n, f->np.p, f->ni.p, f->gw.p, f->n_dir, 3, fv, f->gvel.p);
     launch_ns_assemble(s, f->dev(xs));
-    ctx->launches += 8;
+    ctx->launches += 7;
     f->pat->version++;
     CK(cudaGetLastError());
     return VFV_OK;
@@ -287,12 +298,22 @@ int vfv_flow_create(vfv_ctx* ctx, const vfv_mesh* mh, const double* rho, const d
     CK(f->gcp.upload(L.gcp.data(), L.gcp.size(), s));
     CK(f->gcv.upload(L.gcv.data(), L.gcv.size(), s));
     CK(f->gcc.upload(L.gcc.data(), L.gcc.size(), s));
-    CK(f->trip_ptr.upload(L.trip_ptr.data(), L.trip_ptr.size(), s));
-    CK(f->div_off.upload(L.div_off.data(), L.div_off.size(), s));
-    CK(f->pst_off.upload(L.pst_off.data(), L.pst_off.size(), s));
-    CK(f->sub_off.upload(L.sub_off.data(), L.sub_off.size(), s));
-    CK(f->slot_ptr.upload(L.slot_ptr.data(), L.slot_ptr.size(), s));
-    CK(f->slot_loc.upload(L.slot_loc.data(), L.slot_loc.size(), s));
+    std::vector<int32_t> dloc(n);
+    for (int64_t v = 0; v < n; ++v) {
+        const int32_t* nb = d.nbr_idx.data();
+        dloc[v] = (int32_t)(std::lower_bound(nb + d.nbr_ptr[v], nb + d.nbr_ptr[v + 1], (int32_t)v) - (nb + d.nbr_ptr[v]));
+    }
+    CK(f->dloc.upload(dloc.data(), n, s));
+    CK(f->qlen.upload(L.qlen.data(), n, s));
+    CK(f->qself.upload(L.qself.data(), n, s));
+    CK(f->rself.upload(L.rself.data(), n, s));
+    CK(f->qoff.upload(L.qoff.data(), n + 1, s));
+    CK(f->roff.upload(L.roff.data(), n + 1, s));
+    const NsPlaces* places[6] = {&L.qring, &L.rring, &L.qnb, &L.rgc, &L.rnb, &L.qsub};
+    DBuf<unsigned char>* dst[6] = {&f->qring, &f->rring, &f->qnb, &f->rgc, &f->rnb, &f->qsub};
+    for (int q = 0; q < 6; ++q) CK(dst[q]->upload((const unsigned char*)places[q]->data(), places[q]->bytes(), s));
+    f->wide = L.qring.wide;
+    f->max_len = L.max_len;
     CK(f->den.upload(rho, n, s));
     CK(f->visc.upload(mu, n, s));
     CK(f->fce.upload(fce, 3 * n, s));
@@ -302,7 +323,8 @@ int vfv_flow_create(vfv_ctx* ctx, const vfv_mesh* mh, const double* rho, const d
     CK(f->rc.alloc(n));
     CK(f->mom.alloc(3 * n));
     CK(f->flux.alloc(d.n_dir));
-    CK(f->tv.alloc(f->ntrip));
+    CK(f->gsum.alloc(3 * n));
+    launch_ns_gsum(s, f->dev(nullptr), f->gsum.p);
     CK(f->b.alloc(4 * n));
     CK(f->x.alloc(4 * n));
     CK(f->xu.alloc(4 * n));

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstdlib>
 
 namespace vfv {
 
@@ -66,61 +67,49 @@ void gc_merge(const std::vector<GcEnt>& e, int32_t v, std::vector<int32_t>& stam
 
 int64_t deg(const Dual& d, int64_t v) { return d.nbr_ptr[v + 1] - d.nbr_ptr[v]; }
 
-// Column sequence of row r in push order (appended to out).
-void row_columns(const Dual& d, const NsLayout& L, int64_t r, std::vector<int32_t>& out) {
-    const int64_t N = L.n, P = 3 * N;
-    out.clear();
-    if (r < P) {
-        const int64_t q = r / N, v = r % N;
-        if (v >= L.n_pts) {
-            out.push_back((int32_t)r);
-            return;
-        }
-        for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {  // advection
-            out.push_back((int32_t)(q * N + d.nbr_idx[i]));
-            out.push_back((int32_t)r);
-        }
-        for (int32_t k = L.gcp[v]; k < L.gcp[v + 1]; ++k) out.push_back((int32_t)(P + L.gcv[k]));  // pressure gradient
-        for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {  // diffusion
-            out.push_back((int32_t)(q * N + d.nbr_idx[i]));
-            out.push_back((int32_t)r);
-        }
-        return;
+// Vertices of a set seen once each (stamp[u] == tag), in `out`.
+struct VertexSet {
+    std::vector<int32_t> stamp, out;
+    int32_t tag = 0;
+    explicit VertexSet(int64_t n) : stamp(n, 0) {}
+    void start() {
+        ++tag;
+        out.clear();
     }
-    const int64_t v = r - P;
-    if (v == L.pref_vid) {
-        out.push_back((int32_t)r);
-        return;
+    void add(int32_t u) {
+        if (stamp[u] != tag) {
+            stamp[u] = tag;
+            out.push_back(u);
+        }
     }
-    for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {  // divergence
+};
+
+// Q(v): the vertices of v's p row in the velocity fields (divergence and boundary sub-faces)
+void collect_q(const Dual& d, const NsLayout& L, int64_t v, VertexSet& s) {
+    s.start();
+    s.add((int32_t)v);
+    for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
         const int64_t nb = d.nbr_idx[i];
-        for (int c = 0; c < 3; ++c) {
-            out.push_back((int32_t)(c * N + nb));
-            out.push_back((int32_t)(c * N + v));
-        }
-        for (int64_t k = d.nbr_ptr[v]; k < d.nbr_ptr[v + 1]; ++k)
-            for (int c = 0; c < 3; ++c) {
-                out.push_back((int32_t)(c * N + d.nbr_idx[k]));
-                out.push_back((int32_t)(c * N + v));
-            }
-        for (int64_t k = d.nbr_ptr[nb]; k < d.nbr_ptr[nb + 1]; ++k)
-            for (int c = 0; c < 3; ++c) {
-                out.push_back((int32_t)(c * N + d.nbr_idx[k]));
-                out.push_back((int32_t)(c * N + nb));
-            }
+        s.add((int32_t)nb);
+        for (int64_t k = d.nbr_ptr[nb]; k < d.nbr_ptr[nb + 1]; ++k) s.add(d.nbr_idx[k]);
     }
     if (v >= L.n_pts)
-        for (int64_t b = d.bnd_ptr[v]; b < d.bnd_ptr[v + 1]; ++b) {  // boundary sub-faces of the divergence
-            const int64_t ms[3] = {v, d.bnd_j[b], d.bnd_k[b]};
-            for (int64_t m : ms)
-                for (int c = 0; c < 3; ++c) out.push_back((int32_t)(c * N + m));
+        for (int64_t b = d.bnd_ptr[v]; b < d.bnd_ptr[v + 1]; ++b) {
+            s.add(d.bnd_j[b]);
+            s.add(d.bnd_k[b]);
         }
-    for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {  // pressure stabiliser
+}
+
+// R(v): the vertices of v's p row in the pressure field (stabiliser)
+void collect_r(const Dual& d, const NsLayout& L, int64_t v, VertexSet& s) {
+    s.start();
+    if (d.nbr_ptr[v] == d.nbr_ptr[v + 1]) return;
+    s.add((int32_t)v);
+    for (int32_t k = L.gcp[v]; k < L.gcp[v + 1]; ++k) s.add(L.gcv[k]);
+    for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
         const int64_t nb = d.nbr_idx[i];
-        out.push_back((int32_t)(P + nb));
-        out.push_back((int32_t)r);
-        for (int32_t k = L.gcp[v]; k < L.gcp[v + 1]; ++k) out.push_back((int32_t)(P + L.gcv[k]));
-        for (int32_t k = L.gcp[nb]; k < L.gcp[nb + 1]; ++k) out.push_back((int32_t)(P + L.gcv[k]));
+        s.add((int32_t)nb);
+        for (int32_t k = L.gcp[nb]; k < L.gcp[nb + 1]; ++k) s.add(L.gcv[k]);
     }
 }
 
@@ -162,97 +151,120 @@ std::string build_ns_layout(const Dual& d, int64_t pref_vid, NsLayout& L) {
     L.pref_vid = pref_vid;
     build_grad_coeff(d, L);
     auto gcn = [&](int64_t v) -> int64_t { return L.gcp[v + 1] - L.gcp[v]; };
-    // triplets per row and the per-face block offsets of the p rows
     const int64_t R = 4 * n, P = 3 * n;
-    L.trip_ptr.assign(R + 1, 0);
-    L.div_off.assign(D, 0);
-    L.pst_off.assign(D, 0);
-    L.sub_off.assign(n, 0);
-    std::vector<int64_t> cnt(R, 0);
-#pragma omp parallel for schedule(static)
-    for (int64_t v = 0; v < n; ++v) {
-        const int64_t mom = v < d.n_pts ? 4 * deg(d, v) + gcn(v) : 1;
-        for (int q = 0; q < 3; ++q) cnt[q * n + v] = mom;
-        int64_t off = 0;
-        for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
-            L.div_off[i] = (int32_t)off;
-            off += 6 + 6 * deg(d, v) + 6 * deg(d, d.nbr_idx[i]);
-        }
-        L.sub_off[v] = (int32_t)off;
-        if (v >= d.n_pts) off += 9 * (d.bnd_ptr[v + 1] - d.bnd_ptr[v]);
-        for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
-            L.pst_off[i] = (int32_t)off;
-            off += 2 + gcn(v) + gcn(d.nbr_idx[i]);
-        }
-        cnt[P + v] = v == pref_vid ? 1 : off;
-    }
-    for (int64_t r = 0; r < R; ++r) L.trip_ptr[r + 1] = L.trip_ptr[r] + cnt[r];
-    // Distinct columns of a row are found with a per-thread stamp array over all R columns
-    // (stamp[c] == r: column c already seen in row r); only those are sorted, and a per-thread
-    // position table gives every triplet its slot. A row is handled by one thread, so the stamps
-    // need no reset between rows.
-    // pass 1: distinct columns per row
-    std::vector<int64_t> nz(R, 0);
-#pragma omp parallel
+    // pass 1: triplets, |Q|, |R| and the lengths of the place lists per vertex
+    L.qlen.assign(n, 0);
+    L.qself.assign(n, 0);
+    L.rself.assign(n, 0);
+    L.qoff.assign(n + 1, 0);
+    L.roff.assign(n + 1, 0);
+    std::vector<int32_t> rlen(n, 0);
+    int64_t trips = 0;
+#pragma omp parallel reduction(+ : trips)
     {
-        std::vector<int32_t> seq;
-        std::vector<int32_t> stamp(R, -1);
-#pragma omp for schedule(dynamic, 512)
-        for (int64_t r = 0; r < R; ++r) {
-            row_columns(d, L, r, seq);
-            int64_t k = 0;
-            for (int32_t c : seq)
-                if (stamp[c] != (int32_t)r) {
-                    stamp[c] = (int32_t)r;
-                    ++k;
-                }
-            nz[r] = k;
+        VertexSet set(n);
+#pragma omp for schedule(dynamic, 256)
+        for (int64_t v = 0; v < n; ++v) {
+            trips += 3 * (v < d.n_pts ? 4 * deg(d, v) + gcn(v) : 1);
+            if (v == pref_vid) {
+                trips += 1;
+                continue;
+            }
+            if (v >= d.n_pts) trips += 9 * (d.bnd_ptr[v + 1] - d.bnd_ptr[v]);
+            for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
+                const int64_t nb = d.nbr_idx[i];
+                trips += 6 + 6 * deg(d, v) + 6 * deg(d, nb) + 2 + gcn(v) + gcn(nb);
+                L.qoff[v + 1] += deg(d, nb);
+                L.roff[v + 1] += gcn(nb);
+            }
+            collect_q(d, L, v, set);
+            L.qlen[v] = (int32_t)set.out.size();
+            collect_r(d, L, v, set);
+            rlen[v] = (int32_t)set.out.size();
         }
+    }
+    L.n_trip = trips;
+    for (int64_t v = 0; v < n; ++v) {
+        L.qoff[v + 1] += L.qoff[v];
+        L.roff[v + 1] += L.roff[v];
+        if (v != pref_vid) L.max_len = std::max<int64_t>(L.max_len, std::min<int64_t>(INT_MAX, 3 * (int64_t)L.qlen[v] + rlen[v]));
     }
     L.rp.assign(R + 1, 0);
     int64_t tot = 0;
     for (int64_t r = 0; r < R; ++r) {
-        tot += nz[r];
+        const int64_t v = r % n;
+        if (r < P) tot += v < d.n_pts ? deg(d, v) + 1 + gcn(v) : 1;
+        else tot += v == pref_vid ? 1 : 3 * (int64_t)L.qlen[v] + rlen[v];
         if (tot >= (int64_t)INT_MAX) return "NS pattern too large for 32-bit slot indices";
         L.rp[r + 1] = (int32_t)tot;
     }
-    L.ci.resize(tot);  // ci, slot_ptr and slot_loc are written in full by pass 2
-    L.slot_ptr.resize(tot + 1);
-    L.slot_loc.resize(L.ntrip());
-    L.slot_ptr[tot] = L.ntrip();
-    // pass 2: columns, slots and the push-order triplet lists of every slot
-    std::string err;
+    L.ci.resize(tot);  // ci and the place lists are written in full by pass 2 (but for the reference vertex)
+    const char* force = getenv("VFV_NS_WIDE");  // diagnostics: 32-bit places
+    const bool wide = L.max_len > 65535 || (force && force[0] == '1');
+    const int64_t ng = (int64_t)L.gcv.size(), B = (int64_t)d.bnd_j.size();
+    L.qring.resize(D, wide);
+    L.rring.resize(D, wide);
+    L.qnb.resize(L.qoff[n], wide);
+    L.rgc.resize(ng, wide);
+    L.rnb.resize(L.roff[n], wide);
+    L.qsub.resize(2 * B, wide);
+    // pass 2: columns and places
 #pragma omp parallel
     {
-        std::vector<int32_t> seq, cols, fill;
-        std::vector<int32_t> stamp(R, -1), pos(R, 0);
-#pragma omp for schedule(dynamic, 512)
-        for (int64_t r = 0; r < R; ++r) {
-            row_columns(d, L, r, seq);
-            if ((int64_t)seq.size() != cnt[r]) {
-#pragma omp critical
-                err = "internal: triplet count mismatch";
+        VertexSet set(n);
+        std::vector<int32_t> pos(n, 0);
+#pragma omp for schedule(dynamic, 256)
+        for (int64_t v = 0; v < n; ++v) {
+            for (int q = 0; q < 3; ++q) {  // momentum rows
+                int32_t* c = L.ci.data() + L.rp[q * n + v];
+                if (v >= d.n_pts) {
+                    *c = (int32_t)(q * n + v);
+                    continue;
+                }
+                int64_t i = d.nbr_ptr[v];
+                const int64_t e = d.nbr_ptr[v + 1];
+                for (; i < e && d.nbr_idx[i] < v; ++i) *c++ = (int32_t)(q * n + d.nbr_idx[i]);
+                *c++ = (int32_t)(q * n + v);
+                for (; i < e; ++i) *c++ = (int32_t)(q * n + d.nbr_idx[i]);
+                for (int32_t k = L.gcp[v]; k < L.gcp[v + 1]; ++k) *c++ = (int32_t)(P + L.gcv[k]);
+            }
+            int32_t* c = L.ci.data() + L.rp[P + v];
+            if (v == pref_vid) {
+                *c = (int32_t)(P + v);
                 continue;
             }
-            cols.clear();
-            for (int32_t c : seq)
-                if (stamp[c] != (int32_t)r) {
-                    stamp[c] = (int32_t)r;
-                    cols.push_back(c);
+            collect_q(d, L, v, set);
+            std::sort(set.out.begin(), set.out.end());
+            for (int f = 0; f < 3; ++f)
+                for (int32_t u : set.out) *c++ = (int32_t)(f * n + u);
+            for (size_t t = 0; t < set.out.size(); ++t) pos[set.out[t]] = (int32_t)t;
+            L.qself[v] = pos[v];
+            int64_t o = L.qoff[v];
+            for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
+                const int64_t nb = d.nbr_idx[i];
+                L.qring.set(i, pos[nb]);
+                for (int64_t k = d.nbr_ptr[nb]; k < d.nbr_ptr[nb + 1]; ++k) L.qnb.set(o++, pos[d.nbr_idx[k]]);
+            }
+            if (v >= d.n_pts)
+                for (int64_t b = d.bnd_ptr[v]; b < d.bnd_ptr[v + 1]; ++b) {
+                    L.qsub.set(b, pos[d.bnd_j[b]]);
+                    L.qsub.set(B + b, pos[d.bnd_k[b]]);
                 }
-            std::sort(cols.begin(), cols.end());
-            const int64_t base = L.rp[r];
-            std::copy(cols.begin(), cols.end(), L.ci.begin() + base);
-            for (size_t s = 0; s < cols.size(); ++s) pos[cols[s]] = (int32_t)s;
-            fill.assign(cols.size() + 1, 0);
-            for (int32_t c : seq) fill[pos[c] + 1]++;
-            for (size_t s = 0; s < cols.size(); ++s) fill[s + 1] += fill[s];
-            const int64_t tb = L.trip_ptr[r];
-            for (size_t s = 0; s < cols.size(); ++s) L.slot_ptr[base + s] = tb + fill[s];
-            for (size_t t = 0; t < seq.size(); ++t) L.slot_loc[tb + fill[pos[seq[t]]]++] = (int32_t)t;
+            collect_r(d, L, v, set);
+            std::sort(set.out.begin(), set.out.end());
+            for (int32_t u : set.out) *c++ = (int32_t)(P + u);
+            for (size_t t = 0; t < set.out.size(); ++t) pos[set.out[t]] = (int32_t)t;
+            L.rself[v] = pos[v];
+            o = L.roff[v];
+            for (int32_t k = L.gcp[v]; k < L.gcp[v + 1]; ++k) L.rgc.set(k, pos[L.gcv[k]]);
+            for (int64_t i = d.nbr_ptr[v]; i < d.nbr_ptr[v + 1]; ++i) {
+                const int64_t nb = d.nbr_idx[i];
+                L.rring.set(i, pos[nb]);
+                for (int32_t k = L.gcp[nb]; k < L.gcp[nb + 1]; ++k) L.rnb.set(o++, pos[L.gcv[k]]);
+            }
         }
     }
-    return err;
+    return "";
 }
 
 }  // namespace vfv

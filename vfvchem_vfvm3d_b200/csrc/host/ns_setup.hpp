@@ -1,7 +1,6 @@
 // Symbolic setup of the coupled Navier-Stokes system (SteadyFlow, src/steady/core/steady_flow.rs)
-// on the Voronoi dual: pressure-gradient coefficients, the triplet layout of every row in the
-// reference's push order, and the CSR pattern with the per-slot lists of triplets that the device
-// sums (in push order) into the matrix values.
+// on the Voronoi dual: pressure-gradient coefficients, the CSR pattern of the reference's triplets
+// and, for the pressure rows, the place of every contribution in its row.
 //
 // Unknowns are field-major, [u | v | w | p], n entries each (OperatorBase::add_vecvec_a and
 // friends, src/operator/operator_base.rs:37-94). Every operator of SteadyFlow::assemble_matrix
@@ -14,6 +13,10 @@
 //                           (per face: 2 + |gc v| + |gc n|)
 //   p row of a node:        divergence faces, then 9 per boundary sub-face, then the stabiliser
 //   p row of the reference vertex: the single diagonal (OpSclDomPressureReference drops the rest)
+// So a momentum row holds its own field's {v} and neighbours, then the pressures of grad_coeff(v); a
+// p row holds the same vertices Q(v) (v, its neighbours and theirs) in each of the fields u, v, w and
+// the vertices R(v) (v, its neighbours, grad_coeff(v) and grad_coeff of the neighbours) in the field
+// p, all ascending. The device adds a contribution straight to its place in Q(v) or R(v).
 #pragma once
 #include <cstdint>
 #include <memory>
@@ -45,24 +48,47 @@ struct UninitAlloc : std::allocator<T> {
 template <typename T>
 using uninit_vector = std::vector<T, UninitAlloc<T>>;
 
+// Places within a row, 16 bits each unless some row is longer than that.
+struct NsPlaces {
+    int64_t n = 0;
+    uninit_vector<uint16_t> p16;
+    uninit_vector<uint32_t> p32;
+    bool wide = false;
+    void resize(int64_t count, bool wide_) {
+        n = count;
+        wide = wide_;
+        if (wide) p32.resize(count);
+        else p16.resize(count);
+    }
+    void set(int64_t i, int32_t v) {
+        if (wide) p32[i] = (uint32_t)v;
+        else p16[i] = (uint16_t)v;
+    }
+    const void* data() const { return wide ? (const void*)p32.data() : (const void*)p16.data(); }
+    size_t bytes() const { return (size_t)n * (wide ? 4 : 2); }
+};
+
 struct NsLayout {
-    int64_t n = 0, n_pts = 0, pref_vid = 0;
+    int64_t n = 0, n_pts = 0, pref_vid = 0, n_trip = 0;
     // Tetrahedron::grad_coeff (geom_tet.rs:295-347) as a CSR over vertices, ascending vertex ids
     std::vector<int32_t> gcp;        // [n + 1]
     std::vector<int32_t> gcv;        // [n_gc]
     std::vector<double> gcc;         // [3][n_gc]
-    // triplet layout
-    std::vector<int64_t> trip_ptr;   // [4n + 1] first triplet of every row
-    std::vector<int32_t> div_off;    // [n_dir] offset of face i's divergence block within the p row of its owner
-    std::vector<int32_t> pst_off;    // [n_dir] offset of face i's stabiliser block within that row
-    std::vector<int32_t> sub_off;    // [n] offset of the boundary sub-face block within the p row (nodes)
-    // pattern and slot lists
+    // pattern
     std::vector<int32_t> rp;         // CSR of the 4n x 4n matrix: row pointer [4n + 1]
     uninit_vector<int32_t> ci;       // [nnz] columns
-    uninit_vector<int64_t> slot_ptr; // [nnz + 1] into slot_loc
-    uninit_vector<int32_t> slot_loc; // [ntrip] triplet index within its row, push order per slot
+    // places in the p rows (unset for the reference vertex)
+    int32_t max_len = 0;             // entries of the longest p row
+    std::vector<int32_t> qlen;       // [n] |Q(v)|
+    std::vector<int32_t> qself, rself;    // [n] place of v in Q(v), R(v)
+    std::vector<int64_t> qoff, roff;      // [n + 1] start of v's lists in qnb, rnb
+    NsPlaces qring, rring;           // [n_dir] neighbour i of v in Q(v), R(v)
+    NsPlaces qnb;                    // per face i of v in order: the neighbours of its neighbour, in Q(v)
+    NsPlaces rgc;                    // [n_gc] grad_coeff entries of v in R(v)
+    NsPlaces rnb;                    // per face i of v in order: grad_coeff entries of its neighbour, in R(v)
+    NsPlaces qsub;                   // [2][n_bsub] boundary sub-face vertices j, k in Q(v)
     int64_t nnz() const { return (int64_t)ci.size(); }
-    int64_t ntrip() const { return trip_ptr.empty() ? 0 : trip_ptr.back(); }
+    int64_t ntrip() const { return n_trip; }
 };
 
 // Pressure-gradient coefficients: per vertex, the (vertex, c) pairs of the Green-Gauss gradient

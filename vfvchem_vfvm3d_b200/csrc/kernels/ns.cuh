@@ -1,7 +1,8 @@
 // Device assembly of the coupled Navier-Stokes system (SteadyFlow::assemble_matrix,
 // src/steady/core/steady_flow.rs:255-303) and the flow data it reads (flow_helper.rs:3-179).
-// Compiled with -fmad=false: every value is formed with the reference's operation order and the
-// matrix entries are sums of the row's triplets in push order, as the triplet build does.
+// Compiled with -fmad=false: products and sums round as the reference's scalar code does. Sums over
+// a vertex's faces are split over lanes; a p row's entries are the reference's triplets summed per face,
+// with the terms that all faces of a vertex share (its own gradient weights) collected first.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -24,18 +25,22 @@ struct NsDev {
     const double* x;                               // [u | v | w | p]
     const double *gvel, *gden, *gvisc, *gfce;      // [9][n], [3][n], [3][n], [9][n]
     double *rc, *mom, *flux;                       // [n], [3][n], [n_dir]
-    // triplet layout and output
-    const int64_t* trip_ptr;
-    const int32_t *div_off, *pst_off, *sub_off;
-    double* tv;
+    // rows and places (NsLayout); place lists hold uint16_t, or uint32_t when `wide`
+    const int32_t* dloc;                           // [n] neighbours below v
+    const double* gsum;                            // [3][n] sum of the gradient weights of v
+    const int32_t *qlen, *qself, *rself;
+    const int64_t *qoff, *roff;
+    const void *qring, *rring, *qnb, *rgc, *rnb, *qsub;
+    int wide, max_len;
     double* b;                                     // [4n]
     const int32_t* rp;
-    const int64_t* slot_ptr;
-    const int32_t* slot_loc;
     double* val;
 };
 
-// rc, mom, flux (update_flow / update_flux), then triplet values, b, and the matrix values
+// gsum from the gradient weights (once per mesh)
+void launch_ns_gsum(cudaStream_t s, const NsDev& D, double* gsum);
+
+// rc, mom, flux (update_flow / update_flux), then the matrix values and b
 void launch_ns_assemble(cudaStream_t s, const NsDev& D);
 
 // 4x4 block-Jacobi with blocks {v, N+v, 2N+v, 3N+v} of a field-major 4-field system.

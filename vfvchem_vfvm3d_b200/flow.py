@@ -4,7 +4,7 @@
 (src/steady/core/steady_flow.rs:255-303) for a :class:`~vfvchem_vfvm3d_b200.problems.FlowProblem`:
 velocity boundaries on every face and the pressure fixed at one vertex. ``assemble`` forms A(x)
 and b(x) on the GPU (Rhie-Chow flow data of flow_helper.rs, then every operator's triplets summed
-in push order); ``picard`` runs the damped Picard loop of ``SteadyBase::solve``
+into their entries); ``picard`` runs the damped Picard loop of ``SteadyBase::solve``
 (src/steady/steady_base.rs:70-112) with the GMRES of :class:`~vfvchem_vfvm3d_b200.Pattern`
 (GMRES(100) + 4x4 block-Jacobi by default) as the linear solver.
 """
