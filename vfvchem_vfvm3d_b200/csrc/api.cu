@@ -38,6 +38,59 @@ std::string& vfv_thread_error() {
     return e;
 }
 
+// ================================================================ sliced sparse rows
+void SellHost::build(int64_t n_, const int32_t* rp) {
+    n = n_;
+    const int64_t win = (n + kSellWindow - 1) / kSellWindow, positions = win * kSellWindow;
+    p8.resize(positions);
+    r8.resize(positions);
+    std::vector<int32_t> w(positions / 32);
+    auto len = [&](int64_t r) { return r < n ? rp[r + 1] - rp[r] : 0; };
+    int64_t tails = 0;
+#pragma omp parallel for schedule(static) reduction(+ : tails)
+    for (int64_t b = 0; b < win; ++b) {
+        const int64_t r0 = b * kSellWindow;
+        int32_t ord[kSellWindow];
+        for (int q = 0; q < kSellWindow; ++q) ord[q] = q;
+        std::stable_sort(ord, ord + kSellWindow, [&](int32_t x, int32_t y) { return len(r0 + x) > len(r0 + y); });
+        for (int q = 0; q < kSellWindow; ++q) {
+            p8[r0 + q] = (uint8_t)ord[q];
+            r8[r0 + ord[q]] = (uint8_t)q;
+        }
+        for (int sl = 0; sl < kSellWindow / 32; ++sl) {
+            int64_t sum = 0;
+            for (int q = 0; q < 32; ++q) sum += len(r0 + ord[32 * sl + q]);
+            const int32_t most = len(r0 + ord[32 * sl]);
+            const int32_t wd = (int32_t)std::min<int64_t>(most, 2 * ((sum + 31) / 32) + 8);
+            w[r0 / 32 + sl] = wd;
+            for (int q = 0; q < 32; ++q) tails += std::max(0, len(r0 + ord[32 * sl + q]) - wd);
+        }
+    }
+    so.assign(positions / 32 + 1, 0);
+    int64_t tot = 0;
+    for (int32_t wd : w) tot += 32 * (int64_t)wd;
+    if (tot + tails > INT32_MAX) {  // more slots than 32-bit indices allow: every row in the tail
+        std::fill(w.begin(), w.end(), 0);
+        tails = rp[n];
+    }
+    tot = 0;
+    for (size_t sl = 0; sl < w.size(); ++sl) {
+        tot += 32 * (int64_t)w[sl];
+        so[sl + 1] = (int32_t)tot;
+    }
+    first_tail = tot;
+    tail.clear();
+    if (tails > 0) {
+        tail.resize(n + 1);
+        for (int64_t r = 0; r < n; ++r) {
+            tail[r] = (int32_t)tot;
+            tot += std::max(0, len(r) - width(r));
+        }
+        tail[n] = (int32_t)tot;
+    }
+    slots = tot;
+}
+
 // ================================================================ GMRES driver
 namespace {
 
@@ -526,101 +579,105 @@ DBuf<T>& of_prec(DBuf<double>& d, DBuf<float>& f) {
     else return f;
 }
 
-// Compact triangles of the factor for the Jacobi-sweep apply (k_ilu0_sweep): structure once per
+// Triangles of the factor for the Jacobi-sweep apply (k_ilu0_sweep): structure once per
 // ILU structure (host), values per factor refresh and precision (device). The natural ordering is
 // swept in A's own numbering (A's rows with the factor's values scattered back to A's slots), the
 // multicolour ordering in its factor's permuted numbering.
+int build_split(vfv_ctx* ctx, vfv_pattern* p, IluStruct& S) {
+    cudaStream_t s = ctx->stream;
+    const int64_t n = p->n, nnz = p->nnz;
+    IluStruct::Split& X = S.split;
+    // the factor's structure in its numbering
+    std::vector<int32_t> rp, ci, dg(n);
+    if (S.order == VFV_ILU_NATURAL) {
+        rp = p->h_rp;
+        ci = p->h_ci;
+#pragma omp parallel for schedule(static)
+        for (int64_t i = 0; i < n; ++i)
+            dg[i] = (int32_t)(std::lower_bound(ci.begin() + rp[i], ci.begin() + rp[i + 1], (int32_t)i) - ci.begin());
+    } else {
+        rp.resize(n + 1);
+        ci.resize(nnz);
+        CK(cudaMemcpyAsync(rp.data(), S.rp.p, (n + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(ci.data(), S.ci.p, nnz * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(dg.data(), S.dg.p, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+    }
+    int64_t maxd = 0;
+#pragma omp parallel for schedule(static) reduction(max : maxd)
+    for (int64_t r = 0; r < n; ++r)
+        for (int32_t k = rp[r]; k < rp[r + 1]; ++k) maxd = std::max<int64_t>(maxd, std::abs((int64_t)ci[k] - r));
+    // 16-bit column offsets when the factor's bandwidth allows
+    X.delta16 = maxd <= 32767;
+    for (int up = 0; up < 2; ++up) {
+        IluStruct::Tri& T = up ? X.u : X.l;
+        std::vector<int32_t> tp(n + 1, 0);
+        for (int64_t r = 0; r < n; ++r) tp[r + 1] = tp[r] + (up ? rp[r + 1] - dg[r] - 1 : dg[r] - rp[r]);
+        SellHost h;
+        h.build(n, tp.data());
+        std::vector<int16_t> cd(X.delta16 ? h.slots : 0, 0);
+        std::vector<int32_t> cc(X.delta16 ? 0 : h.slots, -1);
+#pragma omp parallel for schedule(static)
+        for (int64_t r = 0; r < n; ++r) {
+            const int32_t b = up ? dg[r] + 1 : rp[r], cnt = tp[r + 1] - tp[r];
+            for (int32_t q = 0; q < cnt; ++q) {
+                if (X.delta16) cd[h.slot(r, q)] = (int16_t)(ci[b + q] - r);
+                else cc[h.slot(r, q)] = ci[b + q];
+            }
+        }
+        CK(T.sell.upload(h, s));
+        if (X.delta16) CK(T.cd.upload(cd.data(), cd.size(), s));
+        else CK(T.ci.upload(cc.data(), cc.size(), s));
+    }
+    X.built = true;
+    return VFV_OK;
+}
+
 template <typename T>
 int ilu_split_refresh(vfv_ctx* ctx, vfv_pattern* p, IluStruct& S, bool half = false) {
     cudaStream_t s = ctx->stream;
     const int64_t n = p->n, nnz = p->nnz;
     IluStruct::Split& X = S.split;
-    const bool nat = S.order == VFV_ILU_NATURAL;
     if (!X.built) {
-        // the factor's structure in its numbering F
-        std::vector<int32_t> rp, ci, dg(n);
-        if (nat) {
-            rp = p->h_rp;
-            ci = p->h_ci;
-            for (int64_t i = 0; i < n; ++i)
-                for (int32_t k = rp[i]; k < rp[i + 1]; ++k)
-                    if (ci[k] == i) dg[i] = k;
-        } else {
-            rp.resize(n + 1);
-            ci.resize(nnz);
-            CK(cudaMemcpyAsync(rp.data(), S.rp.p, (n + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(ci.data(), S.ci.p, nnz * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(dg.data(), S.dg.p, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-        }
-        int64_t maxd = 0;
-        for (int64_t r = 0; r < n; ++r)
-            for (int32_t k = rp[r]; k < rp[r + 1]; ++k) maxd = std::max<int64_t>(maxd, std::abs((int64_t)ci[k] - r));
-        // 16-bit column offsets when the factor's bandwidth allows. (A reverse Cuthill-McKee
-        // renumbering to make them fit on wider patterns was measured slower on the 10^6-row heat
-        // factor: the sweeps are latency-bound, and renumbered gathers lose the mesh order's locality.)
-        X.delta16 = maxd <= 32767;
-        std::vector<int32_t> lrp(n + 1, 0), urp(n + 1, 0), lc, uc;
-        lc.reserve(nnz / 2);
-        uc.reserve(nnz / 2);
-        for (int64_t r = 0; r < n; ++r) {
-            for (int32_t k = rp[r]; k < rp[r + 1]; ++k) {
-                if (k < dg[r]) lc.push_back(ci[k]);
-                else if (k > dg[r]) uc.push_back(ci[k]);
-            }
-            lrp[r + 1] = (int32_t)lc.size();
-            urp[r + 1] = (int32_t)uc.size();
-        }
-        CK(X.lrp.upload(lrp.data(), n + 1, s));
-        CK(X.urp.upload(urp.data(), n + 1, s));
-        if (X.delta16) {
-            std::vector<int16_t> ld(lc.size()), ud(uc.size());
-            for (int64_t r = 0; r < n; ++r) {
-                for (int32_t k = lrp[r]; k < lrp[r + 1]; ++k) ld[k] = (int16_t)(lc[k] - r);
-                for (int32_t k = urp[r]; k < urp[r + 1]; ++k) ud[k] = (int16_t)(uc[k] - r);
-            }
-            CK(X.lcd.upload(ld.data(), ld.size(), s));
-            CK(X.ucd.upload(ud.data(), ud.size(), s));
-        } else {
-            CK(X.lci.upload(lc.data(), lc.size(), s));
-            CK(X.uci.upload(uc.data(), uc.size(), s));
-        }
-        X.built = true;
+        const int rc = build_split(ctx, p, S);
+        if (rc) return rc;
     }
     constexpr bool dbl = std::is_same<T, double>::value;
     uint64_t& ver = dbl ? X.version64 : X.version32;
-    const int64_t nlow = X.delta16 ? (int64_t)X.lcd.n : (int64_t)X.lci.n, nup = X.delta16 ? (int64_t)X.ucd.n : (int64_t)X.uci.n;
     if (ver != p->version) {
-    const T* lu = of_prec<T>(S.lu64, S.lu32).p;
-    const int32_t *rp = S.rp.p, *dg = S.dg.p;
-    if (nat) {  // the factor's values back in A's slot order
-        DBuf<T>& nv = of_prec<T>(S.nat64, S.nat32);
-        if (!nv.p) CK(nv.alloc(nnz));
-        k_scatter_vals<T><<<grid_for(nnz), 256, 0, s>>>(nnz, S.src.p, lu, nv.p);
+        const T* lu = of_prec<T>(S.lu64, S.lu32).p;
+        const int32_t *rp = S.rp.p, *dg = S.dg.p;
+        if (S.order == VFV_ILU_NATURAL) {  // the factor's values back in A's slot order
+            DBuf<T>& nv = of_prec<T>(S.nat64, S.nat32);
+            if (!nv.p) CK(nv.alloc(nnz));
+            k_scatter_vals<T><<<grid_for(nnz), 256, 0, s>>>(nnz, S.src.p, lu, nv.p);
+            ctx->launches += 1;
+            lu = nv.p;
+            rp = p->rp.p;
+            dg = p->diag_pos.p;
+        }
+        DBuf<T>& dv = of_prec<T>(X.d64, X.d32);
+        if (!dv.p) CK(dv.alloc(n));
+        for (IluStruct::Tri* t : {&X.l, &X.u}) {
+            DBuf<T>& v = of_prec<T>(t->v64, t->v32);
+            if (v.p) continue;
+            CK(v.alloc(std::max<int64_t>(t->sell.slots, 1)));
+            CK(cudaMemsetAsync(v.p, 0, v.n * sizeof(T), s));  // padding stays zero
+        }
+        k_split_vals<T><<<grid_for(n), 256, 0, s>>>((int32_t)n, rp, dg, lu, X.l.sell.dev(), X.u.sell.dev(), of_prec<T>(X.l.v64, X.l.v32).p,
+                                                    of_prec<T>(X.u.v64, X.u.v32).p, dv.p);
         ctx->launches += 1;
-        lu = nv.p;
-        rp = p->rp.p;
-        dg = p->diag_pos.p;
-    }
-    DBuf<T>& lv = of_prec<T>(X.lv64, X.lv32);
-    DBuf<T>& uv = of_prec<T>(X.uv64, X.uv32);
-    DBuf<T>& dv = of_prec<T>(X.d64, X.d32);
-    if (!lv.p) CK(lv.alloc(std::max<int64_t>(nlow, 1)));
-    if (!uv.p) CK(uv.alloc(std::max<int64_t>(nup, 1)));
-    if (!dv.p) CK(dv.alloc(n));
-    k_split_vals<T><<<grid_for(n), 256, 0, s>>>((int32_t)n, rp, dg, lu, X.lrp.p, X.urp.p, lv.p, uv.p, dv.p);
-    ctx->launches += 1;
-    CK(cudaGetLastError());
-    ver = p->version;
+        CK(cudaGetLastError());
+        ver = p->version;
     }
     if constexpr (!dbl) {  // the row-scaled half copies of the float values, when asked for
         if (half && X.version_half != p->version) {
-            if (!X.lvh.p) CK(X.lvh.alloc(std::max<int64_t>(nlow, 1)));
-            if (!X.uvh.p) CK(X.uvh.alloc(std::max<int64_t>(nup, 1)));
-            if (!X.lsc.p) CK(X.lsc.alloc(n));
-            if (!X.usc.p) CK(X.usc.alloc(n));
-            k_half_rows<<<grid_for(n), 256, 0, s>>>((int32_t)n, X.lrp.p, X.lv32.p, reinterpret_cast<__half*>(X.lvh.p), X.lsc.p);
-            k_half_rows<<<grid_for(n), 256, 0, s>>>((int32_t)n, X.urp.p, X.uv32.p, reinterpret_cast<__half*>(X.uvh.p), X.usc.p);
+            for (IluStruct::Tri* t : {&X.l, &X.u}) {
+                if (!t->vh.p) CK(t->vh.alloc(std::max<int64_t>(t->sell.slots, 1)));
+                if (!t->sc.p) CK(t->sc.alloc(n));
+                k_half_rows<<<grid_for(n, kSellWindow), kSellWindow, 0, s>>>((int32_t)n, t->sell.dev(), t->v32.p,
+                                                                            reinterpret_cast<__half*>(t->vh.p), t->sc.p);
+            }
             ctx->launches += 2;
             CK(cudaGetLastError());
             X.version_half = p->version;
@@ -629,76 +686,69 @@ int ilu_split_refresh(vfv_ctx* ctx, vfv_pattern* p, IluStruct& S, bool half = fa
     return VFV_OK;
 }
 
-// Operands of the Jacobi-sweep apply, from the refreshed compact triangles.
+// Operands of the Jacobi-sweep apply, from the refreshed triangles.
 template <typename T>
 struct SweepOps {
+    struct Tri {
+        SellDev sell{};
+        const void* cols = nullptr;
+        const T* v = nullptr;
+        // float factors only: the row-scaled half-precision values and their row scales (vfv_gmres_opts::ilu_sweep_half)
+        const __half* vh = nullptr;
+        const float* sc = nullptr;
+    };
     int32_t n = 0;
-    int lanes = 4;  // lanes per row (measured on the 10^6-row heat factor: 1 for float values, 2 for double)
     bool delta16 = false;
-    const int32_t *lrp = nullptr, *urp = nullptr, *perm = nullptr;
-    const void *lcols = nullptr, *ucols = nullptr;
-    const T *lv = nullptr, *uv = nullptr, *d = nullptr;
-    // float factors only: the row-scaled half-precision values and their row scales (vfv_gmres_opts::ilu_sweep_half)
-    const __half *lvh = nullptr, *uvh = nullptr;
-    const float *lsc = nullptr, *usc = nullptr;
+    Tri l, u;
+    const int32_t* perm = nullptr;
+    const T* d = nullptr;
 };
 
 template <typename T>
 SweepOps<T> sweep_ops(const vfv_pattern* p, IluStruct& S, bool half = false) {
     IluStruct::Split& X = S.split;
     SweepOps<T> o;
-    if (half && std::is_same<T, float>::value) {
-        o.lvh = reinterpret_cast<const __half*>(X.lvh.p);
-        o.uvh = reinterpret_cast<const __half*>(X.uvh.p);
-        o.lsc = X.lsc.p;
-        o.usc = X.usc.p;
-    }
     o.n = (int32_t)p->n;
-    o.lanes = std::is_same<T, double>::value ? 2 : 1;
-    if (const char* e = getenv("VFV_SWEEP_LANES")) {
-        const int g = std::atoi(e);
-        if (g == 1 || g == 2 || g == 4 || g == 8) o.lanes = g;
-    }
     o.delta16 = X.delta16;
-    o.lrp = X.lrp.p;
-    o.urp = X.urp.p;
-    o.lcols = X.delta16 ? (const void*)X.lcd.p : (const void*)X.lci.p;
-    o.ucols = X.delta16 ? (const void*)X.ucd.p : (const void*)X.uci.p;
-    o.lv = of_prec<T>(X.lv64, X.lv32).p;
-    o.uv = of_prec<T>(X.uv64, X.uv32).p;
+    for (int up = 0; up < 2; ++up) {
+        IluStruct::Tri& t = up ? X.u : X.l;
+        typename SweepOps<T>::Tri& q = up ? o.u : o.l;
+        q.sell = t.sell.dev();
+        q.cols = X.delta16 ? (const void*)t.cd.p : (const void*)t.ci.p;
+        q.v = of_prec<T>(t.v64, t.v32).p;
+        if (half && std::is_same<T, float>::value) {
+            q.vh = reinterpret_cast<const __half*>(t.vh.p);
+            q.sc = t.sc.p;
+        }
+    }
     o.d = of_prec<T>(X.d64, X.d32).p;
     o.perm = S.order == VFV_ILU_NATURAL ? nullptr : S.perm.p;
     return o;
 }
 
-
-template <typename T, typename TC, bool LOWER, int G>
-cudaError_t launch_sweep_g(cudaLaunchConfig_t& cfg, const SweepOps<T>& o, const T* rhs, const T* prev, T* next, T* w0, T* out,
+template <typename T, typename TC, bool LOWER, bool TAIL>
+cudaError_t launch_sweep_c(cudaLaunchConfig_t& cfg, const SweepOps<T>& o, const T* rhs, const T* prev, T* next, T* w0, T* out,
                            const DevStatus* st) {
-    cfg.gridDim = dim3((unsigned)grid_for((int64_t)o.n * G, kSwBlock));
+    const typename SweepOps<T>::Tri& t = LOWER ? o.l : o.u;
     if constexpr (std::is_same<T, float>::value) {
-        if (o.lvh)
-            return cudaLaunchKernelEx(&cfg, k_ilu0_sweep<T, TC, LOWER, G, __half>, o.n, LOWER ? o.lrp : o.urp,
-                                      (const TC*)(LOWER ? o.lcols : o.ucols), LOWER ? o.lvh : o.uvh, LOWER ? o.lsc : o.usc, o.d, o.perm,
+        if (t.vh)
+            return cudaLaunchKernelEx(&cfg, k_ilu0_sweep<T, TC, LOWER, TAIL, __half>, o.n, t.sell, (const TC*)t.cols, t.vh, t.sc, o.d, o.perm,
                                       rhs, prev, next, w0, out, st);
     }
-    return cudaLaunchKernelEx(&cfg, k_ilu0_sweep<T, TC, LOWER, G, T>, o.n, LOWER ? o.lrp : o.urp, (const TC*)(LOWER ? o.lcols : o.ucols),
-                              LOWER ? o.lv : o.uv, (const float*)nullptr, o.d, o.perm, rhs, prev, next, w0, out, st);
+    return cudaLaunchKernelEx(&cfg, k_ilu0_sweep<T, TC, LOWER, TAIL, T>, o.n, t.sell, (const TC*)t.cols, t.v, (const float*)nullptr, o.d,
+                              o.perm, rhs, prev, next, w0, out, st);
 }
 
 template <typename T, bool LOWER>
 cudaError_t launch_sweep(cudaLaunchConfig_t& cfg, const SweepOps<T>& o, const T* rhs, const T* prev, T* next, T* w0, T* out,
                          const DevStatus* st) {
-    if (o.delta16) {
-        if (o.lanes == 1) return launch_sweep_g<T, int16_t, LOWER, 1>(cfg, o, rhs, prev, next, w0, out, st);
-        if (o.lanes == 2) return launch_sweep_g<T, int16_t, LOWER, 2>(cfg, o, rhs, prev, next, w0, out, st);
-        if (o.lanes == 8) return launch_sweep_g<T, int16_t, LOWER, 8>(cfg, o, rhs, prev, next, w0, out, st);
-        return launch_sweep_g<T, int16_t, LOWER, 4>(cfg, o, rhs, prev, next, w0, out, st);
-    }
-    if (o.lanes == 1) return launch_sweep_g<T, int32_t, LOWER, 1>(cfg, o, rhs, prev, next, w0, out, st);
-    if (o.lanes == 2) return launch_sweep_g<T, int32_t, LOWER, 2>(cfg, o, rhs, prev, next, w0, out, st);
-    if (o.lanes == 8) return launch_sweep_g<T, int32_t, LOWER, 8>(cfg, o, rhs, prev, next, w0, out, st);
-    return launch_sweep_g<T, int32_t, LOWER, 4>(cfg, o, rhs, prev, next, w0, out, st);
+    cfg.gridDim = dim3((unsigned)grid_for(o.n, kSwBlock));
+    const bool tail = (LOWER ? o.l : o.u).sell.tail != nullptr;
+    if (o.delta16)
+        return tail ? launch_sweep_c<T, int16_t, LOWER, true>(cfg, o, rhs, prev, next, w0, out, st)
+                    : launch_sweep_c<T, int16_t, LOWER, false>(cfg, o, rhs, prev, next, w0, out, st);
+    return tail ? launch_sweep_c<T, int32_t, LOWER, true>(cfg, o, rhs, prev, next, w0, out, st)
+                : launch_sweep_c<T, int32_t, LOWER, false>(cfg, o, rhs, prev, next, w0, out, st);
 }
 
 // z = M^-1 r by `sweeps` Jacobi sweeps of the lower and `usweeps` of the upper ILU(0) factor: one

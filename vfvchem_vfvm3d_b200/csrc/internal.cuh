@@ -89,6 +89,58 @@ struct DBuf {  // device buffer, freed with its owner
 inline int grid_for(int64_t threads, int block = 256) { return (int)std::max<int64_t>(1, (threads + block - 1) / block); }
 
 
+// ================================================================ sliced sparse rows
+// A sparse matrix's rows in slices of 32 for one thread per row: entry q of the 32 rows of a slice is
+// 32 consecutive slots, so a warp reads its indices and values in full lines. (A thread per row of a
+// CSR array makes every warp load touch one line per few rows, and the L1's wavefronts, not HBM,
+// bound the kernel.) Within each window of kSellWindow rows the rows are sorted by length, so the 32
+// rows of a slice have nearly equal lengths (7-8% padding on the triangles of the 10^6-row heat
+// matrix, 47% unsorted). A slice is as wide as its longest row, but at most twice its mean plus 8:
+// entries past that width are kept row by row after the slices (tail), so that a few long rows cannot
+// blow up the storage.
+constexpr int kSellWindow = 256;
+
+struct SellHost {
+    int64_t n = 0, slots = 0, first_tail = 0;
+    std::vector<int32_t> so;    // [positions / 32 + 1] first slot of each slice
+    std::vector<uint8_t> p8;    // [positions] offset in the window of the row at this position
+    std::vector<uint8_t> r8;    // [positions] position in the window of this row
+    std::vector<int32_t> tail;  // [n + 1] slots of a row's entries past its slice's width; empty: no such row
+    int32_t width(int64_t row) const {
+        const int64_t s = pos(row) >> 5;
+        return (so[s + 1] - so[s]) >> 5;
+    }
+    int64_t pos(int64_t row) const { return (row & ~(int64_t)(kSellWindow - 1)) + r8[row]; }
+    int64_t slot(int64_t row, int32_t q) const {
+        const int64_t p = pos(row);
+        const int32_t w = width(row);
+        return q < w ? (int64_t)so[p >> 5] + 32 * (int64_t)q + (p & 31) : (int64_t)tail[row] + (q - w);
+    }
+    void build(int64_t n_, const int32_t* rp);  // from the row lengths rp[i + 1] - rp[i]
+};
+
+struct SellDev {
+    const int32_t* so;
+    const uint8_t* p8;
+    const uint8_t* r8;
+    const int32_t* tail;  // null: no tails
+};
+
+struct SellBuf {
+    DBuf<int32_t> so, tail;
+    DBuf<uint8_t> p8, r8;
+    int64_t slots = 0;
+    cudaError_t upload(const SellHost& h, cudaStream_t s) {
+        slots = h.slots;
+        cudaError_t e = so.upload(h.so.data(), h.so.size(), s);
+        if (e == cudaSuccess) e = p8.upload(h.p8.data(), h.p8.size(), s);
+        if (e == cudaSuccess) e = r8.upload(h.r8.data(), h.r8.size(), s);
+        if (e == cudaSuccess) e = tail.upload(h.tail.data(), h.tail.size(), s);
+        return e;
+    }
+    SellDev dev() const { return {so.p, p8.p, r8.p, tail.p}; }
+};
+
 // ================================================================ ILU structure (host-built)
 struct IluStruct {
     int order = -1;
@@ -121,18 +173,23 @@ struct IluStruct {
     } chain[2];                     // [0] double, [1] float
 
     // Jacobi-sweep applies (vfv_gmres_opts::ilu_sweeps): the factor's strictly lower and strictly
-    // upper parts as compact CSR arrays and its diagonal, in A's own numbering for the natural
+    // upper parts in sliced layouts and its diagonal, in A's own numbering for the natural
     // ordering (nat64/nat32 hold the factor's values scattered back to A's slots) and in the
     // factor's permuted numbering for the multicolour one
+    struct Tri {
+        SellBuf sell;
+        DBuf<int16_t> cd;     // columns as offsets from the row (Split::delta16; 0: padding)
+        DBuf<int32_t> ci;     // absolute columns (-1: padding)
+        DBuf<double> v64;
+        DBuf<float> v32;
+        DBuf<uint16_t> vh;    // half-precision copies of v32 divided by their row scales
+        DBuf<float> sc;       // row scales: the largest magnitude of the row in the triangle
+    };
     struct Split {
         bool built = false, delta16 = false;  // delta16: columns stored as int16 offsets from the row
-        DBuf<int32_t> lrp, urp;
-        DBuf<int16_t> lcd, ucd;
-        DBuf<int32_t> lci, uci;
-        DBuf<double> lv64, uv64, d64;
-        DBuf<float> lv32, uv32, d32;
-        DBuf<uint16_t> lvh, uvh;  // half-precision copies of lv32 / uv32 divided by their row scales
-        DBuf<float> lsc, usc;     // row scales: the largest magnitude of the row in each triangle
+        Tri l, u;
+        DBuf<double> d64;
+        DBuf<float> d32;
         uint64_t version64 = ~0ull, version32 = ~0ull, version_half = ~0ull;
     } split;
     DBuf<double> nat64;

@@ -11,7 +11,7 @@
 // Storage (permuted numbering): CSR lu_rp/lu_ci with columns ascending, lu_diag[i] = slot of the
 // diagonal. Lower part = slots before lu_diag (unit diagonal implied), upper = from lu_diag on.
 #pragma once
-#include "../common.cuh"
+#include "../internal.cuh"
 
 #include <cuda_fp16.h>
 
@@ -380,14 +380,27 @@ __global__ void __launch_bounds__(kLevBlock, kLevMinBlocks) k_ilu0_level(int32_t
 // over all rows (an SpMV over one triangle) instead of one latency-bound launch per level; the
 // operator is linear and fixed, so flexible and plain GMRES both accept it.
 //
-// Storage: N and S as separate compact CSR arrays (a sweep streams only its own triangle's bytes;
-// inside A's rows the two halves share DRAM sectors), columns as 16-bit offsets from the row when
-// the pattern's bandwidth allows (TC = int16_t; int32_t absolute columns otherwise), and D apart.
-// G lanes per row, sweep_k(G) entries per lane loaded before the programmatic-dependent-launch wait (the
-// factor does not change between sweeps); lane partial sums are combined by a butterfly (fixed order).
-constexpr int kSwBlock = 256;
-__host__ __device__ constexpr int sweep_k(int G) { return G >= 4 ? 2 : 8 / G; }  // ~8 entries of a row held before the wait
+// Storage: N and S apart (a sweep streams only its own triangle's bytes; inside A's rows the two
+// halves share DRAM sectors) in the sliced layout (SellDev), a thread per row; columns as 16-bit
+// offsets from the row when the factor's bandwidth allows (TC = int16_t, 0: padding; int32_t absolute
+// columns otherwise, -1: padding), and D apart. sweep_k entries per thread are loaded before the
+// programmatic-dependent-launch wait (the factor does not change between sweeps). Per row the entries
+// are summed in column order; padding is skipped, not multiplied.
+// Measured on the 10^6-row heat factor, apply of 4 + 4 sweeps, rows walked in CSR arrays before and
+// now: half values 131.7 -> 113.8 us, float 140.9 ->
+// 123.2, double (two lanes a row before) 230 -> 227 with 4 entries in flight (238 and 245 with 8 at 5 and 4
+// blocks per SM).
+constexpr int kSwBlock = kSellWindow;
+template <typename T>
+__host__ __device__ constexpr int sweep_k() {
+    return sizeof(T) == 4 ? 8 : 4;
+}
 
+template <typename TC>
+__device__ __forceinline__ bool sweep_has(TC c) {
+    if constexpr (sizeof(TC) == 2) return c != 0;
+    else return c >= 0;
+}
 template <typename TC>
 __device__ __forceinline__ int32_t sweep_col(TC c, int32_t row) {
     if constexpr (sizeof(TC) == 2) return row + (int32_t)c;
@@ -405,69 +418,81 @@ __device__ __forceinline__ T sweep_val(T v) {
 }
 __device__ __forceinline__ float sweep_val(__half v) { return __half2float(v); }
 
-template <typename T, typename TC, bool LOWER, int G, typename TV = T>
-__global__ void __launch_bounds__(kSwBlock) k_ilu0_sweep(int32_t n, const int32_t* __restrict__ rowp, const TC* __restrict__ cols,
-                                                         const TV* __restrict__ val, const float* __restrict__ rs, const T* __restrict__ d,
-                                                         const int32_t* __restrict__ perm, const T* rhs, const T* prev, T* next, T* w0,
-                                                         T* out, const DevStatus* __restrict__ st) {
-    const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int32_t i = (int32_t)(gt / G);
-    const int lane = (int)(gt & (G - 1));
-    int32_t kb = 0, ke = 0;
-    constexpr int kSwK = sweep_k(G);
-    int32_t c[kSwK];
-    T v[kSwK];
+// TAIL: some rows have entries past their slice's width. (A template argument: the branch alone kept
+// the right-hand side's load behind the gathers, 6 us per apply.)
+template <typename T, typename TC, bool LOWER, bool TAIL, typename TV = T>
+__global__ void __launch_bounds__(kSwBlock, 8)
+    k_ilu0_sweep(int32_t n, SellDev S, const TC* __restrict__ cols, const TV* __restrict__ val, const float* __restrict__ rs,
+                 const T* __restrict__ d, const int32_t* __restrict__ perm, const T* rhs, const T* prev, T* next, T* w0, T* out,
+                 const DevStatus* st) {
+    constexpr int K = sweep_k<T>();
+    const int32_t t = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     // done is set once and for all within a cycle: a launch after it loads nothing (12 us of loads
     // per launch on 10^6 rows otherwise, for the steps left in a cycle graph's group)
     const bool skip = st && st->done;
-    if (i < n) {
-        kb = __ldg(rowp + i);
-        ke = __ldg(rowp + i + 1);
-    }
-    if (skip) ke = kb;
+    const int32_t k0 = __ldg(S.so + (t >> 5)), k1 = __ldg(S.so + (t >> 5) + 1);
+    const int32_t i = (t & ~(kSellWindow - 1)) + (int32_t)__ldg(S.p8 + t);
+    const int32_t kb = k0 + (t & 31), w = skip ? 0 : (k1 - k0) >> 5;
+    TC c[K];
+    TV v[K];
 #pragma unroll
-    for (int q = 0; q < kSwK; ++q) {
-        const int32_t k = kb + lane + q * G;
-        c[q] = k < ke ? sweep_col<TC>(__ldg(cols + k), i) : -1;
-        v[q] = k < ke ? (T)sweep_val(__ldg(val + k)) : T(0);
+    for (int q = 0; q < K; ++q) {
+        c[q] = q < w ? __ldg(cols + kb + 32 * q) : (sizeof(TC) == 2 ? TC(0) : TC(-1));
+        v[q] = q < w ? __ldg(val + kb + 32 * q) : TV(0.f);
     }
     pdl_launch_dependents();
     pdl_wait();
     if (skip || (st && st->done)) return;
     T s = T(0);
 #pragma unroll
-    for (int q = 0; q < kSwK; ++q)
-        if (c[q] >= 0) s += v[q] * prev[c[q]];
-    for (int32_t k = kb + lane + kSwK * G; k < ke; k += G) s += (T)sweep_val(__ldg(val + k)) * prev[sweep_col<TC>(__ldg(cols + k), i)];
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-    if (i >= n || lane != 0) return;
-    if (rs) s *= (T)__ldg(rs + i);
-    if (LOWER) {
-        const T u = rhs[i] - s;
-        next[i] = u;
-        if (w0) w0[i] = u / __ldg(d + i);
-    } else {
-        const T w = (rhs[i] - s) / __ldg(d + i);
-        if (out) out[perm ? __ldg(perm + i) : i] = w;
-        else next[i] = w;
+    for (int q = 0; q < K; ++q)
+        if (sweep_has(c[q])) s += (T)sweep_val(v[q]) * prev[sweep_col(c[q], i)];
+#pragma unroll 2
+    for (int q = K; q < w; ++q) {
+        const TC cq = __ldg(cols + kb + 32 * q);
+        const TV vq = __ldg(val + kb + 32 * q);  // beside the column, not after the test of it
+        if (sweep_has(cq)) s += (T)sweep_val(vq) * prev[sweep_col(cq, i)];
+    }
+    if (TAIL && i < n)
+        for (int32_t k = __ldg(S.tail + i); k < __ldg(S.tail + i + 1); ++k) s += (T)sweep_val(__ldg(val + k)) * prev[sweep_col(__ldg(cols + k), i)];
+    if (i < n) {
+        const T u = rhs[i] - (rs ? s * (T)__ldg(rs + i) : s);
+        if (LOWER) {
+            next[i] = u;
+            if (w0) w0[i] = u / __ldg(d + i);
+        } else {
+            const T x = u / __ldg(d + i);
+            if (out) out[perm ? __ldg(perm + i) : i] = x;
+            else next[i] = x;
+        }
     }
 }
 
-// Values of the compact triangles from the factor's rows (thread per row): the strictly lower
-// entries of row i to lv[lrp[i]..], the strictly upper ones to uv[urp[i]..], the diagonal to dv[i].
+// slot of a row's entries in a sliced layout: base + 32 q for q < w, then from `tail`
+struct SellRow {
+    int32_t base, w, tail;
+};
+__device__ __forceinline__ SellRow sell_row(const SellDev& S, int32_t i) {
+    const int32_t p = (i & ~(kSellWindow - 1)) + (int32_t)__ldg(S.r8 + i);
+    const int32_t k0 = __ldg(S.so + (p >> 5)), k1 = __ldg(S.so + (p >> 5) + 1);
+    return {k0 + (p & 31), (k1 - k0) >> 5, S.tail ? __ldg(S.tail + i) : 0};
+}
+
+// Values of the triangles from the factor's rows (thread per row): the strictly lower entries of row
+// i to lv, the strictly upper ones to uv, the diagonal to dv[i].
 template <typename T>
-__global__ void k_split_vals(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ dg, const T* __restrict__ lu,
-                             const int32_t* __restrict__ lrp, const int32_t* __restrict__ urp, T* __restrict__ lv, T* __restrict__ uv,
-                             T* __restrict__ dv) {
+__global__ void k_split_vals(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ dg, const T* __restrict__ lu, SellDev L,
+                             SellDev U, T* __restrict__ lv, T* __restrict__ uv, T* __restrict__ dv) {
     const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
     const int32_t b = rp[i], dd = dg[i], e = rp[i + 1];
-    int32_t o = lrp[i];
-    for (int32_t k = b; k < dd; ++k) lv[o++] = lu[k];
+    const SellRow l = sell_row(L, i), u = sell_row(U, i);
+    for (int32_t k = b; k < dd; ++k) lv[k - b < l.w ? l.base + 32 * (k - b) : l.tail + (k - b - l.w)] = lu[k];
     dv[i] = lu[dd];
-    o = urp[i];
-    for (int32_t k = dd + 1; k < e; ++k) uv[o++] = lu[k];
+    for (int32_t k = dd + 1; k < e; ++k) {
+        const int32_t q = k - dd - 1;
+        uv[q < u.w ? u.base + 32 * q : u.tail + (q - u.w)] = lu[k];
+    }
 }
 
 // y[i] = in[perm[i]]: the right-hand side in the factor's numbering (first step of a sweep apply)
@@ -478,19 +503,22 @@ __global__ void k_perm_gather(int32_t n, const int32_t* __restrict__ perm, const
     if (i < n) y[i] = in[__ldg(perm + i)];
 }
 
-// Half-precision copies of the compact triangles' float values, row-scaled: scale[i] = the row's
-// largest magnitude in the triangle (1 for an empty or all-zero row), h[k] = half(v[k] / scale[i])
+// Half-precision copies of a triangle's float values, row-scaled: scale[i] = the row's largest
+// magnitude in the triangle (1 for an empty or all-zero row), h[k] = half(v[k] / scale[i])
 // rounded to nearest, so every stored value lies in [-1, 1] whatever the matrix's scaling.
-__global__ void k_half_rows(int32_t n, const int32_t* __restrict__ rowp, const float* __restrict__ v, __half* __restrict__ h,
-                            float* __restrict__ scale) {
-    const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= n) return;
-    const int32_t b = rowp[i], e = rowp[i + 1];
+__global__ void __launch_bounds__(kSellWindow) k_half_rows(int32_t n, SellDev S, const float* __restrict__ v, __half* __restrict__ h,
+                                                           float* __restrict__ scale) {
+    const int32_t t = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int32_t i = (t & ~(kSellWindow - 1)) + (int32_t)__ldg(S.p8 + t);
+    const int32_t k0 = __ldg(S.so + (t >> 5)), w = (__ldg(S.so + (t >> 5) + 1) - k0) >> 5, kb = k0 + (t & 31);
+    const int32_t t0 = S.tail && i < n ? S.tail[i] : 0, t1 = S.tail && i < n ? S.tail[i + 1] : 0;
     float m = 0.f;
-    for (int32_t k = b; k < e; ++k) m = fmaxf(m, fabsf(v[k]));
+    for (int q = 0; q < w; ++q) m = fmaxf(m, fabsf(v[kb + 32 * q]));
+    for (int32_t k = t0; k < t1; ++k) m = fmaxf(m, fabsf(v[k]));
     const float sc = m > 0.f ? m : 1.f;
-    scale[i] = sc;
-    for (int32_t k = b; k < e; ++k) h[k] = __float2half_rn(v[k] / sc);
+    if (i < n) scale[i] = sc;
+    for (int q = 0; q < w; ++q) h[kb + 32 * q] = __float2half_rn(v[kb + 32 * q] / sc);
+    for (int32_t k = t0; k < t1; ++k) h[k] = __float2half_rn(v[k] / sc);
 }
 
 // Factor values back in A's own slot order (natural ordering): out[src[k]] = lu[k].
