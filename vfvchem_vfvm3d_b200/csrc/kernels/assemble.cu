@@ -13,7 +13,7 @@
 // off-diagonal coefficients are written straight into their CSR slots and lane 0 of the group adds
 // the diagonal contributions in the same order, so the result is deterministic and atomic-free.
 // This file is compiled with -fmad=false: every product and sum rounds exactly like the
-// reference's scalar code.
+// reference's scalar code (the transport diagonal's sums are split over a row's lanes).
 #include "assemble.cuh"
 
 namespace vfv {
@@ -132,29 +132,6 @@ __global__ void __launch_bounds__(256, 6) k_assemble_heat(HeatDev H) {
 }
 
 // ---------------------------------------------------------------- transient transport (batched meshes)
-// Face mass flux with zero pressure and body force (flow_helper.rs:72-179 with vel_rc = 0):
-//   F = rho_f (u_f . n) A,  rho = 1,  u_f = skew-corrected arithmetic mean of the vertex velocities.
-__global__ void __launch_bounds__(256) k_face_flux(TransportDev T) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= T.n) return;
-    const int64_t N = T.n, D = T.n_dir;
-    const double uv = T.vel[v], vv = T.vel[N + v], wv = T.vel[2 * N + v];
-    double g[9];
-    for (int c = 0; c < 9; ++c) g[c] = T.gvel[c * N + v];
-    for (int32_t i = T.np[v]; i < T.np[v + 1]; ++i) {
-        const int32_t nb = T.ni[i];
-        const double sx = T.skew[i], sy = T.skew[D + i], sz = T.skew[2 * D + i];
-        const double nx = T.norm[i], ny = T.norm[D + i], nz = T.norm[2 * D + i];
-        const double den_f = 0.5 * (1.0 + 1.0) + 0.5 * (sx * (0.0 + 0.0) + sy * (0.0 + 0.0) + sz * (0.0 + 0.0));
-        const double u_f = 0.5 * (uv + T.vel[nb]) + 0.5 * (sx * (g[0] + T.gvel[nb]) + sy * (g[1] + T.gvel[N + nb]) + sz * (g[2] + T.gvel[2 * N + nb]));
-        const double v_f = 0.5 * (vv + T.vel[N + nb]) +
-                           0.5 * (sx * (g[3] + T.gvel[3 * N + nb]) + sy * (g[4] + T.gvel[4 * N + nb]) + sz * (g[5] + T.gvel[5 * N + nb]));
-        const double w_f = 0.5 * (wv + T.vel[2 * N + nb]) +
-                           0.5 * (sx * (g[6] + T.gvel[6 * N + nb]) + sy * (g[7] + T.gvel[7 * N + nb]) + sz * (g[8] + T.gvel[8 * N + nb]));
-        T.flux[i] = den_f * (u_f * nx + v_f * ny + w_f * nz + 0.0) * T.area[i];
-    }
-}
-
 // power-law factor A(|Pe|) = max(0, 1 - 0.1 |Pe|)^5, the fifth power as x^2 x^2 x
 __device__ __forceinline__ double power_law(double pe) {
     const double x = fmax(1.0 - 0.1 * fabs(pe), 0.0);
@@ -162,43 +139,65 @@ __device__ __forceinline__ double power_law(double pe) {
     return x2 * x2 * x;
 }
 
-// Row v, push order: time (v,v), diffusion (v,n)/(v,v) per face, advection (v,n)/(v,v) per face.
-// Off-diagonal slot = c + coeff, diagonal = -vol/dt - sum c - sum coeff, each summed in that order.
+// Lanes per row of the transport matrix: a row's ~15 faces, two per lane, read in runs of 64 bytes
+constexpr int kRowG = 8;
+
+__device__ __forceinline__ double lanes_sum(double x, unsigned mask) {
+#pragma unroll
+    for (int o = kRowG / 2; o > 0; o >>= 1) x += __shfl_xor_sync(mask, x, o, kRowG);
+    return x;
+}
+
+// Face mass flux with zero pressure and body force (flow_helper.rs:72-179 with vel_rc = 0):
+//   F = rho_f (u_f . n) A,  rho = 1,  u_f = skew-corrected arithmetic mean of the vertex velocities,
+// and the matrix row: time (v,v), diffusion (v,n)/(v,v) per face, advection (v,n)/(v,v) per face, i.e.
+// off-diagonal c + coeff, diagonal -vol/dt - sum c - sum coeff. One pass over the faces, kRowG lanes
+// per row (two kernels with a thread per row walked them three times: 1,450 + 790 us cold for 884,000
+// rows, 525 us now).
 __global__ void __launch_bounds__(256) k_assemble_transport(TransportDev T) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & (kRowG - 1);
+    const int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kRowG;
     if (v >= T.n) return;
     const int64_t N = T.n, E = T.n_dir;
     const int32_t b = T.np[v], e = T.np[v + 1];
     const int32_t rb = T.rp[v], dl = T.dloc[v];
     const double Dv = T.D[v];
     const double gx = T.gD[v], gy = T.gD[N + v], gz = T.gD[2 * N + v];
-    double diag = -T.cvol[v] / T.dt;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int32_t i = b; i < e; ++i) {
-            const int32_t nb = T.ni[i];
-            const double Dn = T.D[nb];
-            const double sx = T.skew[i], sy = T.skew[E + i], sz = T.skew[2 * E + i];
-            const double dm = (Dv + Dn != 0.0) ? 2.0 * Dv * Dn / (Dv + Dn) : 0.0;
-            double df = dm + 0.5 * (sx * (gx + T.gD[nb]) + sy * (gy + T.gD[N + nb]) + sz * (gz + T.gD[2 * N + nb]));
-            df = df > 0.0 ? df : dm;
-            const double cond = df * T.area[i] / T.dist[i];
-            const int32_t loc = i - b;
-            const int32_t slot = rb + loc + (loc >= dl ? 1 : 0);
-            if (pass == 0) {
-                T.val[slot] = cond;
-                diag += -cond;
-            } else {
-                const double wgt_f = 0.5 * (1.0 + 1.0) + 0.5 * (sx * (0.0 + 0.0) + sy * (0.0 + 0.0) + sz * (0.0 + 0.0));
-                const double den_f = wgt_f;
-                const double flux = den_f != 0.0 ? wgt_f / den_f * T.flux[i] : 0.0;
-                const double pe = cond != 0.0 ? flux / cond : 0.0;
-                const double coeff = cond * (power_law(pe) - 1.0) + fmax(-flux, 0.0);
-                T.val[slot] += coeff;
-                diag += -coeff;
-            }
-        }
+    const double uv = T.vel[v], vv = T.vel[N + v], wv = T.vel[2 * N + v];
+    double g[9];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) g[c] = T.gvel[c * N + v];
+    double dif = 0.0, adv = 0.0;
+    for (int32_t i = b + lane; i < e; i += kRowG) {
+        const int32_t nb = T.ni[i];
+        const double sx = T.skew[i], sy = T.skew[E + i], sz = T.skew[2 * E + i];
+        const double nx = T.norm[i], ny = T.norm[E + i], nz = T.norm[2 * E + i];
+        const double area = T.area[i];
+        const double wgt_f = 0.5 * (1.0 + 1.0) + 0.5 * (sx * (0.0 + 0.0) + sy * (0.0 + 0.0) + sz * (0.0 + 0.0));
+        const double u_f = 0.5 * (uv + T.vel[nb]) + 0.5 * (sx * (g[0] + T.gvel[nb]) + sy * (g[1] + T.gvel[N + nb]) + sz * (g[2] + T.gvel[2 * N + nb]));
+        const double v_f = 0.5 * (vv + T.vel[N + nb]) +
+                           0.5 * (sx * (g[3] + T.gvel[3 * N + nb]) + sy * (g[4] + T.gvel[4 * N + nb]) + sz * (g[5] + T.gvel[5 * N + nb]));
+        const double w_f = 0.5 * (wv + T.vel[2 * N + nb]) +
+                           0.5 * (sx * (g[6] + T.gvel[6 * N + nb]) + sy * (g[7] + T.gvel[7 * N + nb]) + sz * (g[8] + T.gvel[8 * N + nb]));
+        const double face = wgt_f * (u_f * nx + v_f * ny + w_f * nz + 0.0) * area;
+        T.flux[i] = face;
+        const double Dn = T.D[nb];
+        const double dm = (Dv + Dn != 0.0) ? 2.0 * Dv * Dn / (Dv + Dn) : 0.0;
+        double df = dm + 0.5 * (sx * (gx + T.gD[nb]) + sy * (gy + T.gD[N + nb]) + sz * (gz + T.gD[2 * N + nb]));
+        df = df > 0.0 ? df : dm;
+        const double cond = df * area / T.dist[i];
+        const double flux = wgt_f != 0.0 ? wgt_f / wgt_f * face : 0.0;
+        const double pe = cond != 0.0 ? flux / cond : 0.0;
+        const double coeff = cond * (power_law(pe) - 1.0) + fmax(-flux, 0.0);
+        const int32_t loc = i - b;
+        T.val[rb + loc + (loc >= dl ? 1 : 0)] = cond + coeff;
+        dif += -cond;
+        adv += -coeff;
     }
-    T.val[rb + dl] = diag;
+    const unsigned mask = group_mask(kRowG);
+    dif = lanes_sum(dif, mask);
+    adv = lanes_sum(adv, mask);
+    if (lane == 0) T.val[rb + dl] = -T.cvol[v] / T.dt + dif + adv;
 }
 
 // b = -c_prev vol / dt  (OpSclDomTimeUnity::apply_time right-hand side; zero-flux walls add nothing)
@@ -266,9 +265,8 @@ void launch_transport_dAdD_dot(cudaStream_t s, const TransportDev& T, const doub
     k_transport_dAdD_dot<<<(unsigned)((T.n + 255) / 256), 256, 0, s>>>(T, lam, c, part, counter, out);
 }
 
-void launch_face_flux(cudaStream_t s, const TransportDev& T) { k_face_flux<<<(unsigned)((T.n + 255) / 256), 256, 0, s>>>(T); }
 void launch_assemble_transport(cudaStream_t s, const TransportDev& T) {
-    k_assemble_transport<<<(unsigned)((T.n + 255) / 256), 256, 0, s>>>(T);
+    k_assemble_transport<<<(unsigned)((T.n * kRowG + 255) / 256), 256, 0, s>>>(T);
 }
 void launch_transport_rhs(cudaStream_t s, int64_t n, const double* cvol, double dt, const double* c_prev, double* b) {
     k_transport_rhs<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, cvol, dt, c_prev, b);

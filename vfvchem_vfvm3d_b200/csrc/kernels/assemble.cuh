@@ -59,12 +59,11 @@ struct TransportDev {
     const double* gD;       // [3][n] its gradient
     const double* vel;      // [3][n] velocity
     const double* gvel;     // [9][n] its gradient (du/dx, du/dy, du/dz, dv/dx, ...)
-    double* flux;           // [n_dir] face mass flux (density 1)
+    double* flux;           // [n_dir] face mass flux (density 1), written by launch_assemble_transport
     double dt;
     double* val;            // [nnz]
 };
 
-void launch_face_flux(cudaStream_t s, const TransportDev& T);
 void launch_assemble_transport(cudaStream_t s, const TransportDev& T);
 void launch_transport_rhs(cudaStream_t s, int64_t n, const double* cvol, double dt, const double* c_prev, double* b);
 

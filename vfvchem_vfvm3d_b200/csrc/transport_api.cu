@@ -165,9 +165,8 @@ int vfv_transport_assemble(vfv_ctx* ctx, vfv_transport* t, const double* D, cons
     const double* f4[4] = {t->fields.p, t->fields.p + n, t->fields.p + 2 * n, t->fields.p + 3 * n};
     launch_grad(s, n, t->np.p, t->ni.p, t->gw.p, t->n_dir, 4, f4, t->grads.p);
     const TransportDev T = t->dev();
-    launch_face_flux(s, T);
     launch_assemble_transport(s, T);
-    ctx->launches += 3;
+    ctx->launches += 2;
     CK(cudaGetLastError());
     t->pat->version++;
     return VFV_OK;
