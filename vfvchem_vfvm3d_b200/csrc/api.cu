@@ -539,7 +539,7 @@ int ilu_refresh(vfv_ctx* ctx, vfv_pattern* p, IluStruct& S, bool want32, long lo
 
 // z = (LU)^-1 r: one launch per level, lower levels then upper levels in reverse, chained with
 // programmatic dependent launch. `in` and `out` may alias; `t` must not alias either.
-template <typename T, bool LOWER>
+template <typename T, bool LOWER, bool LAST = false>
 cudaError_t launch_level(cudaStream_t s, const IluStruct& S, int l, bool pdl, const T* lu, const T* in, T* t, T* out, const DevStatus* st,
                          int prio = 0, bool use_prio = false) {
     const int32_t r0 = S.lev_ptr[l], r1 = S.lev_ptr[l + 1];
@@ -561,15 +561,16 @@ cudaError_t launch_level(cudaStream_t s, const IluStruct& S, int l, bool pdl, co
     }
     cfg.attrs = na ? attr : nullptr;
     cfg.numAttrs = na;
-    return cudaLaunchKernelEx(&cfg, k_ilu0_level<T, LOWER>, r0, r1, (const int32_t*)S.rp.p, (const int32_t*)S.ci.p, (const int32_t*)S.dg.p, lu,
+    return cudaLaunchKernelEx(&cfg, k_ilu0_level<T, LOWER, LAST>, r0, r1, (const int32_t*)S.rp.p, (const int32_t*)S.ci.p, (const int32_t*)S.dg.p, lu,
                               (const int32_t*)S.perm.p, in, t, out, st);
 }
 
 template <typename T>
 void ilu_apply_levels(cudaStream_t s, const IluStruct& S, const T* lu, const T* in, T* t, T* out, const DevStatus* st, int prio = 0,
                       bool use_prio = false) {
-    for (int l = 0; l < S.nlev; ++l) launch_level<T, true>(s, S, l, l > 0, lu, in, t, out, st, prio, use_prio);
-    for (int l = S.nlev - 1; l >= 0; --l) launch_level<T, false>(s, S, l, true, lu, in, t, out, st, prio, use_prio);
+    for (int l = 0; l + 1 < S.nlev; ++l) launch_level<T, true>(s, S, l, l > 0, lu, in, t, out, st, prio, use_prio);
+    launch_level<T, true, true>(s, S, S.nlev - 1, S.nlev > 1, lu, in, t, out, st, prio, use_prio);
+    for (int l = S.nlev - 2; l >= 0; --l) launch_level<T, false>(s, S, l, true, lu, in, t, out, st, prio, use_prio);
 }
 
 // the buffer of precision T out of a double / float pair
@@ -931,7 +932,7 @@ struct Gmres : SolverBase {
     bool pending_steps = false;
     int steps_seen = 0;
     IluStruct* ilu = nullptr;
-    uint64_t bj_version = ~0ull;
+    uint64_t bj_version = ~0ull, valk_version = ~0ull;  // versions of the pattern's values behind binv and valK
     // overlapped engine: preconditioned basis Z, SpMV output a, q = M^-1 a, the second stream
     DBuf<T> Zb, abuf, qbuf;
     DBuf<double> coefz;
@@ -1534,7 +1535,9 @@ struct Gmres : SolverBase {
             if (rc) return rc;
         }
         // matrix preparation for this solve
-        if (precond == VFV_PRECOND_JACOBI) {
+        if (valK.p && valk_version == p->version) {
+            // the Krylov copy of the values is of this matrix already (time steps, adjoint solves)
+        } else if (precond == VFV_PRECOND_JACOBI) {
             k_jacobi_inv<<<grid_for(n), 256, 0, s>>>(n, p->diag_pos.p, p->val.p, dinv.p);
             k_scale_cols<T><<<grid_for(p->nnz), 256, 0, s>>>(p->nnz, p->ci.p, p->val.p, dinv.p, valK.p);
             ctx->launches += 2;
@@ -1542,6 +1545,7 @@ struct Gmres : SolverBase {
             k_scale_cols<T><<<grid_for(p->nnz), 256, 0, s>>>(p->nnz, p->ci.p, p->val.p, nullptr, valK.p);
             ctx->launches += 1;
         }
+        valk_version = p->version;
         if (precond == VFV_PRECOND_ILU0) {
             int rc = ilu_refresh(ctx, p, *ilu, mixed, wait_polls);
             if (!rc && sweeps > 0) rc = ilu_split_refresh<T>(ctx, p, *ilu, sweep_half);
@@ -2156,7 +2160,7 @@ int vfv_ilu0_apply_device(vfv_ctx* ctx, vfv_pattern* p, int ilu_order, const dou
     int rc = ilu_for_apply<double>(ctx, p, ilu_order, &S);
     if (rc) return rc;
     ilu_apply_levels<double>(ctx->stream, *S, S->lu64.p, r, reinterpret_cast<double*>(S->chain[0].work.p), z, nullptr);
-    ctx->launches += 2 * S->nlev;
+    ctx->launches += 2 * S->nlev - 1;
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
     if (levels) *levels = S->nlev;
@@ -2174,7 +2178,7 @@ int vfv_ilu0_apply_device_f32(vfv_ctx* ctx, vfv_pattern* p, int ilu_order, const
     int rc = ilu_for_apply<float>(ctx, p, ilu_order, &S);
     if (rc) return rc;
     ilu_apply_levels<float>(ctx->stream, *S, S->lu32.p, r, t, z, nullptr);
-    ctx->launches += 2 * S->nlev;
+    ctx->launches += 2 * S->nlev - 1;
     CK(cudaGetLastError());
     if (levels) *levels = S->nlev;
     return VFV_OK;
@@ -2257,7 +2261,7 @@ int vfv_ilu0_apply_device_noalloc(vfv_ctx* ctx, vfv_pattern* p, int ilu_order, c
     int rc = ilu_refresh(ctx, p, S, false, 0, false);  // numeric factor into the storage made at set-up
     if (rc) return rc;
     ilu_apply_levels<double>(ctx->stream, S, S.lu64.p, r, scratch, z, nullptr);
-    ctx->launches += 2 * S.nlev;
+    ctx->launches += 2 * S.nlev - 1;
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
     if (levels) *levels = S.nlev;
