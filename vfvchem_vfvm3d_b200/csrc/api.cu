@@ -906,7 +906,9 @@ VecShape vec_shape(int64_t rows) {
 // the launches they save, 130 against 118 ms at 131,072 rows).
 constexpr int kFoldMax = 128;
 
-constexpr int kStepsPerIf = 4;  // Arnoldi steps per IF node of a cycle graph
+constexpr int kStepsPerIf = 4;   // Arnoldi steps per IF node of a cycle graph
+constexpr int kMaxGraphs = 6;     // cycle graphs of one solver
+constexpr int kWantedOften = 6;   // cycles that would have used a graph before it is built
 
 // Sets the IF condition of the next group of Arnoldi steps of a cycle graph: run it unless the solve stopped.
 __global__ void k_step_condition(cudaGraphConditionalHandle h, const DevStatus* st) { cudaGraphSetConditional(h, st->done ? 0u : 1u); }
@@ -927,10 +929,15 @@ struct Gmres : SolverBase {
     DBuf<unsigned> counter;
     DBuf<DevStatus> st;
     KrylovDev K{};
-    cudaGraphExec_t exec = nullptr;
-    int64_t graph_nodes = 0, step_nodes = 0;
-    bool pending_steps = false;
-    int steps_seen = 0;
+    // Cycle graphs by the number of leading steps that run unconditionally (CycleGraph), the steps that
+    // each cycle of the last solve took, and how often a graph was wanted that is not built
+    struct CycleGraph {
+        cudaGraphExec_t exec = nullptr;
+        int64_t nodes = 0, step_nodes = 0;  // kernels of the unconditional part, of one conditional step
+    };
+    std::map<int, CycleGraph> graphs;
+    std::map<int, int> wanted;
+    std::vector<int> last_cycles;
     IluStruct* ilu = nullptr;
     uint64_t bj_version = ~0ull, valk_version = ~0ull;  // versions of the pattern's values behind binv and valK
     // overlapped engine: preconditioned basis Z, SpMV output a, q = M^-1 a, the second stream
@@ -959,7 +966,8 @@ struct Gmres : SolverBase {
     std::vector<MeshStat> mesh_stat;  // per-mesh state after the last solve
     long long wait_polls = kDefaultWaitPolls;  // bounded device waits of this solve (vfv_gmres_opts::wait_limit)
     ~Gmres() override {
-        if (exec) cudaGraphExecDestroy(exec);
+        for (auto& g : graphs)
+            if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (s2) cudaStreamDestroy(s2);
@@ -1422,14 +1430,6 @@ struct Gmres : SolverBase {
         k_residual<T, G><<<sp_blocks, kBlk, 0, s>>>(K, p->rp.p, p->ci.p, p->val.p, x.p, b.p, V.p);
     }
 
-    // The whole cycle, captured as one straight graph (every step's kernels return at once once the
-    // device `done` flag is set).
-    void enqueue_cycle(cudaStream_t s, vfv_pattern* p) {
-        enqueue_prologue(s);
-        for (int j = 0; j < m; ++j) enqueue_step(s, p, j);
-        enqueue_epilogue(s, p);
-    }
-
     // Appends what `fn` enqueues on s to graph g after the nodes `deps`; returns the new frontier.
     template <typename F>
     cudaError_t capture_into(cudaStream_t s, cudaGraph_t g, std::vector<cudaGraphNode_t>& deps, F fn) {
@@ -1457,49 +1457,67 @@ struct Gmres : SolverBase {
         return cudaSuccess;
     }
 
-    // The cycle as a graph whose Arnoldi steps sit in IF nodes, kStepsPerIf steps per node: a
-    // one-thread kernel before each node sets the condition from the device `done` flag, so the
-    // groups after convergence cost one tiny launch each instead of ~25 kernels per step (a step of
-    // a running group that finds the solve done still returns at once, as in the straight graph). Returns an error (and leaves no graph) where the
-    // CUDA driver cannot build it; the caller then captures the straight graph.
-    cudaError_t build_conditional_graph(cudaStream_t s, vfv_pattern* p, cudaGraph_t* out, int64_t* top_nodes, int64_t* step_nodes) {
+    // Appends to graph g, after `deps`, a condition kernel and an IF node whose body `fill` builds: run
+    // unless the solve stopped. deps becomes the IF node.
+    template <typename F>
+    cudaError_t add_if(cudaStream_t s, cudaGraph_t g, std::vector<cudaGraphNode_t>& deps, F fill) {
+        cudaGraphConditionalHandle h;  // one handle per conditional node
+        cudaError_t e = cudaGraphConditionalHandleCreate(&h, g, 1u, cudaGraphCondAssignDefault);
+        if (e == cudaSuccess) e = capture_into(s, g, deps, [&] { k_step_condition<<<1, 1, 0, s>>>(h, st.p); });
+        if (e != cudaSuccess) return e;
+        cudaGraphNodeParams np{};
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = h;
+        np.conditional.type = cudaGraphCondTypeIf;
+        np.conditional.size = 1;
+        cudaGraphNode_t cn;
+        e = cudaGraphAddNode(&cn, g, deps.empty() ? nullptr : deps.data(), deps.size(), &np);
+        if (e == cudaSuccess) e = fill(np.conditional.phGraph_out[0]);
+        deps.assign(1, cn);
+        return e;
+    }
+
+    // The cycle as a graph: the first `lead` Arnoldi steps as plain nodes, the others in IF nodes,
+    // kStepsPerIf steps per node: a one-thread kernel before each node sets the condition from the
+    // device `done` flag, so the groups after convergence cost one tiny launch each instead of ~25
+    // kernels per step (a step of a running group that finds the solve done still returns at once, as
+    // the plain ones do). Behind leading steps, which are expected to be all, the groups sit in one
+    // more IF node, so that skipping them costs one node. With lead = m there is no conditional node.
+    // Returns an error (and leaves no graph) where the CUDA driver cannot build it.
+    cudaError_t build_cycle_graph(cudaStream_t s, vfv_pattern* p, int lead, cudaGraph_t* out, int64_t* top_nodes, int64_t* step_nodes) {
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaGraphCreate(&g, 0);
         if (e != cudaSuccess) return e;
         std::vector<cudaGraphNode_t> deps;
         int64_t body_nodes = 0;
-        const char* stage = "prologue";
-        e = capture_into(s, g, deps, [&] { enqueue_prologue(s); });
-        for (int j0 = 0; j0 < m && e == cudaSuccess; j0 += kStepsPerIf) {
-            const int j1 = std::min(m, j0 + kStepsPerIf);
-            stage = "handle";  // one handle per conditional node
-            cudaGraphConditionalHandle h;
-            e = cudaGraphConditionalHandleCreate(&h, g, 1u, cudaGraphCondAssignDefault);
-            if (e != cudaSuccess) break;
-            stage = "condition kernel";
-            e = capture_into(s, g, deps, [&] { k_step_condition<<<1, 1, 0, s>>>(h, st.p); });
-            if (e != cudaSuccess) break;
-            stage = "conditional node";
-            cudaGraphNodeParams np{};
-            np.type = cudaGraphNodeTypeConditional;
-            np.conditional.handle = h;
-            np.conditional.type = cudaGraphCondTypeIf;
-            np.conditional.size = 1;
-            cudaGraphNode_t cn;
-            e = cudaGraphAddNode(&cn, g, deps.empty() ? nullptr : deps.data(), deps.size(), &np);
-            if (e != cudaSuccess) break;
-            cudaGraph_t body = np.conditional.phGraph_out[0];
-            std::vector<cudaGraphNode_t> none;
-            stage = "step body";
-            e = capture_into(s, body, none, [&] {
-                for (int j = j0; j < j1; ++j) enqueue_step(s, p, j);
-            });
-            if (e == cudaSuccess && j0 == 0) {
-                size_t bn = 0;
-                e = cudaGraphGetNodes(body, nullptr, &bn);
-                body_nodes = (int64_t)bn / (j1 - j0);
+        auto groups = [&](cudaGraph_t to, std::vector<cudaGraphNode_t>& dp) {
+            cudaError_t r = cudaSuccess;
+            for (int j0 = lead; j0 < m && r == cudaSuccess; j0 += kStepsPerIf) {
+                const int j1 = std::min(m, j0 + kStepsPerIf);
+                r = add_if(s, to, dp, [&](cudaGraph_t body) {
+                    std::vector<cudaGraphNode_t> none;
+                    cudaError_t q = capture_into(s, body, none, [&] {
+                        for (int j = j0; j < j1; ++j) enqueue_step(s, p, j);
+                    });
+                    size_t bn = 0;
+                    if (q == cudaSuccess && j0 == lead) q = cudaGraphGetNodes(body, nullptr, &bn);
+                    if (j0 == lead) body_nodes = (int64_t)bn / (j1 - j0);
+                    return q;
+                });
             }
-            deps.assign(1, cn);
+            return r;
+        };
+        const char* stage = "prologue";
+        e = capture_into(s, g, deps, [&] {
+            enqueue_prologue(s);
+            for (int j = 0; j < lead; ++j) enqueue_step(s, p, j);
+        });
+        if (e == cudaSuccess && lead < m) {
+            stage = "conditional steps";
+            e = lead == 0 ? groups(g, deps) : add_if(s, g, deps, [&](cudaGraph_t body) {
+                std::vector<cudaGraphNode_t> none;
+                return groups(body, none);
+            });
         }
         if (e == cudaSuccess) {
             stage = "epilogue";
@@ -1507,7 +1525,7 @@ struct Gmres : SolverBase {
         }
         if (e != cudaSuccess) {
             if (const char* t = getenv("VFV_TRACE_SOLVE"))
-                if (t[0] == '1') fprintf(stderr, "[vfv] conditional cycle graph not built (%s, %zu dependencies): %s\n", stage, deps.size(), cudaGetErrorString(e));
+                if (t[0] == '1') fprintf(stderr, "[vfv] cycle graph not built (%s, %zu dependencies): %s\n", stage, deps.size(), cudaGetErrorString(e));
             cudaGraphDestroy(g);
             cudaGetLastError();
             return e;
@@ -1518,6 +1536,45 @@ struct Gmres : SolverBase {
         *top_nodes = (int64_t)tn;
         *step_nodes = body_nodes;
         return cudaSuccess;
+    }
+
+    // captures, instantiates and keeps the cycle graph with `lead` unconditional steps
+    int add_graph(vfv_ctx* ctx, vfv_pattern* p, int lead) {
+        cudaGraph_t graph = nullptr;
+        CycleGraph g;
+        cudaError_t e = build_cycle_graph(ctx->stream, p, lead, &graph, &g.nodes, &g.step_nodes);
+        if (e == cudaSuccess) {
+            e = cudaGraphInstantiate(&g.exec, graph, 0);
+            cudaGraphDestroy(graph);
+        }
+        if (e != cudaSuccess) {
+            if (const char* t = getenv("VFV_TRACE_SOLVE"))
+                if (t[0] == '1') fprintf(stderr, "[vfv] cycle graph with %d leading steps not built: %s\n", lead, cudaGetErrorString(e));
+            cudaGetLastError();
+            return set_err(ctx, VFV_CUDA_ERROR, std::string("cycle graph: ") + cudaGetErrorString(e));
+        }
+        graphs.emplace(lead, g);
+        return VFV_OK;
+    }
+
+    // The graph of the next cycle. An IF node costs ~12 us whether its steps run or not (3 us per
+    // Arnoldi step: 3.70 against 3.23 ms for 150 steps on 8,000 rows with none), so the steps that a
+    // cycle is expected to take anyway - as many as the same cycle of the last solve took, or all m
+    // after a full cycle - run unconditionally. Which graph runs never changes a result: a step after
+    // convergence does nothing. A graph takes milliseconds to build, so one is added only when it has
+    // been wanted kWantedOften times, at most kMaxGraphs per solver; otherwise the one with the most
+    // leading steps up to the expected number is taken.
+    void pick_graph(vfv_ctx* ctx, vfv_pattern* p, int cycle, const std::vector<int>& took, const CycleGraph** out, int* lead) {
+        int want = 0;
+        if (cycle < (int)last_cycles.size()) want = last_cycles[cycle];
+        else if (!took.empty() && took.back() >= m) want = m;
+        want = std::max(0, std::min(want, m));
+        if (graphs.begin()->first == 0 && want > 0 && !graphs.count(want) && (int)graphs.size() < kMaxGraphs && ++wanted[want] == kWantedOften)
+            add_graph(ctx, p, want);  // where it cannot be built the others serve
+        auto it = graphs.upper_bound(want);
+        if (it != graphs.begin()) --it;  // straight graphs only: the first one
+        *lead = it->first;
+        *out = &it->second;
     }
 
     // A batched solver (nm > 0, a block-diagonal system of independent meshes) runs one Krylov
@@ -1605,46 +1662,24 @@ struct Gmres : SolverBase {
             k_residual<T, G><<<grid_for(n * G), kBlk, 0, s>>>(K, p->rp.p, p->ci.p, p->val.p, x.p, b.p, V.p);
             ctx->launches += 1;
         }
-        if (engine != VFV_ENGINE_PERSISTENT && !exec) {
-            cudaGraph_t graph = nullptr;
-            cudaError_t e = cudaErrorUnknown;
-            if (!getenv("VFV_STRAIGHT_GRAPH")) {  // conditional steps unless asked for the straight graph
-                e = build_conditional_graph(s, p, &graph, &graph_nodes, &step_nodes);
-                if (e == cudaSuccess) {
-                    e = cudaGraphInstantiate(&exec, graph, 0);
-                    cudaGraphDestroy(graph);
-                    if (e != cudaSuccess) {
-                        if (const char* t = getenv("VFV_TRACE_SOLVE"))
-                            if (t[0] == '1') fprintf(stderr, "[vfv] conditional cycle graph not instantiated: %s\n", cudaGetErrorString(e));
-                        exec = nullptr;
-                        cudaGetLastError();
-                    }
-                }
-            }
-            if (e != cudaSuccess) {
-                step_nodes = 0;
-                CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-                enqueue_cycle(s, p);
-                CK(cudaStreamEndCapture(s, &graph));
-                size_t nodes = 0;
-                CK(cudaGraphGetNodes(graph, nullptr, &nodes));
-                graph_nodes = (int64_t)nodes;
-                e = cudaGraphInstantiate(&exec, graph, 0);
-                cudaGraphDestroy(graph);
-                CK(e);
-            }
+        if (engine != VFV_ENGINE_PERSISTENT && graphs.empty()) {
+            // conditional steps unless asked for the straight graph or refused by the driver
+            int rc = getenv("VFV_STRAIGHT_GRAPH") ? VFV_CUDA_ERROR : add_graph(ctx, p, 0);
+            if (rc) rc = add_graph(ctx, p, m);
+            if (rc) return rc;
         }
-        int cycles = 0, rc = VFV_OK;
-        steps_seen = 0;
-        pending_steps = false;
+        int cycles = 0, rc = VFV_OK, steps_seen = 0;
+        std::vector<int> took;            // steps of this solve's cycles
+        const CycleGraph* ran = nullptr;  // the last launched cycle's graph and its unconditional steps
+        int ran_lead = 0;
         DevStatus hst{};
         for (;;) {
             CK(cudaMemcpyAsync(ctx->h_status, st.p, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             hst = *ctx->h_status;
-            if (pending_steps) {
-                ctx->launches += step_nodes * (int64_t)(hst.total_steps - steps_seen);
-                pending_steps = false;
+            if (ran) {
+                took.push_back(hst.total_steps - steps_seen);
+                ctx->launches += ran->step_nodes * (int64_t)std::max(0, took.back() - ran_lead);
             }
             steps_seen = hst.total_steps;
             if (hst.timeout) {
@@ -1668,11 +1703,11 @@ struct Gmres : SolverBase {
                 break;
             }
             if (engine != VFV_ENGINE_PERSISTENT) {
-                CK(cudaGraphLaunch(exec, s));
-                // straight graph: every node launches; conditional graph: the top-level nodes, plus
-                // the bodies of the steps run (counted when the cycle's status comes back)
-                ctx->launches += graph_nodes;
-                pending_steps = step_nodes > 0;
+                pick_graph(ctx, p, cycles, took, &ran, &ran_lead);
+                CK(cudaGraphLaunch(ran->exec, s));
+                // the top-level nodes, and the bodies of the conditional steps that run (counted when
+                // the cycle's status comes back)
+                ctx->launches += ran->nodes;
             } else {
                 CycleArgs A = cycle_args(p);
                 void* args[] = {&A};
@@ -1681,6 +1716,7 @@ struct Gmres : SolverBase {
             }
             ++cycles;
         }
+        last_cycles.swap(took);
         CK(cudaGetLastError());
         if (trace.p) dump_trace(ctx, cycles);
         if (const char* e = getenv("VFV_PROFILE_STEP")) {
