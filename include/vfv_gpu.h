@@ -152,8 +152,8 @@ int vfv_spmv_device(vfv_ctx* ctx, const vfv_pattern* p, const double* x, double*
 int vfv_spmv_device_f32(vfv_ctx* ctx, vfv_pattern* p, const float* x, float* y);
 /* Autotuner: measures the pattern's SpMV in each of its shapes (2 to 32 lanes per row, 1 to 8 strides
  * of indices and values loaded per lane before the gathers; double and float values) and keeps the
- * fastest for every later SpMV and solver of this pattern; call before its first solve. Returns the
- * chosen lanes (either pointer may be NULL). */
+ * fastest for every later SpMV of this pattern and for solvers of patterns with long rows (solvers
+ * keep short rows in slices of their own); call before its first solve. Returns the chosen lanes (either pointer may be NULL). */
 int vfv_pattern_autotune(vfv_ctx* ctx, vfv_pattern* p, int32_t* lanes64, int32_t* lanes32);
 /* the SpMV shape in use: lanes per row and strides per lane, double and float (pointers may be NULL) */
 int vfv_pattern_spmv_shape(const vfv_pattern* p, int32_t* lanes64, int32_t* strides64, int32_t* lanes32, int32_t* strides32);

@@ -906,6 +906,38 @@ VecShape vec_shape(int64_t rows) {
 // the launches they save, 130 against 118 ms at 131,072 rows).
 constexpr int kFoldMax = 128;
 
+// The sliced rows of a pattern's SpMV: wanted
+//  - for a full wave of the sliced kernel's resident blocks, 148 x 5 x 256 rows: with fewer, a thread
+//    per row leaves the chip idle and several lanes per CSR row are faster (8,000 rows: 3.27 against
+//    3.56 ms per solve; 103,823: 10.1 / 10.4; 125,000 double: 40.9 / 42.4; 262,144 double: 32.8 / 32.4;
+//    10^6 float: 93.0 / 87.7);
+//  - where every row is short and like its neighbours (no tails, no slice wider than kSellMost): a
+//    thread would walk a longer row alone while CSR gives it up to a warp;
+//  - where columns and double values take at most 1/16 of the memory that is free now: the CSR matrix
+//    stays (residuals, factors), so a matrix that nearly fills the device is solved from CSR as it is.
+constexpr int64_t kSellRows = 148 * kSellBlocks * kSellWindow;
+constexpr int32_t kSellMost = 64;
+int build_pattern_sell(vfv_ctx* ctx, vfv_pattern* p) {
+    p->sell_built = true;
+    if (p->n < kSellRows) return VFV_OK;
+    SellHost h;
+    h.build(p->n, p->h_rp.data());
+    int32_t most = 0;
+    for (size_t q = 0; q + 1 < h.so.size(); ++q) most = std::max(most, (h.so[q + 1] - h.so[q]) / 32);
+    if (!h.tail.empty() || most > kSellMost) return VFV_OK;
+    size_t avail = 0, total = 0;
+    CK(cudaMemGetInfo(&avail, &total));
+    if ((size_t)h.slots * (sizeof(int32_t) + sizeof(double)) > avail / 16) return VFV_OK;
+    std::vector<int32_t> ci(std::max<int64_t>(h.slots, 1), -1);
+#pragma omp parallel for schedule(static)
+    for (int64_t r = 0; r < p->n; ++r)
+        for (int32_t q = 0; q < p->h_rp[r + 1] - p->h_rp[r]; ++q) ci[h.slot(r, q)] = p->h_ci[p->h_rp[r] + q];
+    CK(p->sell.upload(h, ctx->stream));
+    CK(p->sell_ci.upload(ci.data(), ci.size(), ctx->stream));
+    p->sell_use = true;
+    return VFV_OK;
+}
+
 constexpr int kStepsPerIf = 4;   // Arnoldi steps per IF node of a cycle graph
 constexpr int kMaxGraphs = 6;     // cycle graphs of one solver
 constexpr int kWantedOften = 6;   // cycles that would have used a graph before it is built
@@ -919,6 +951,7 @@ struct Gmres : SolverBase {
     int m = 0, precond = 0, ilu_order = 0, engine = 0;
     int nblk = 0, mega_grid = 0, mega_chunk = 0;
     VecShape shape = VecShape::wide;  // of the multi-vector kernels
+    bool sell = false;                // valK and the SpMV in the pattern's sliced layout
     DBuf<T> V, z, z2, zc, valK;
     DBuf<unsigned> bar;
     DBuf<unsigned long long> trace;  // per-phase timestamps of the last cycle (VFV_TRACE_CYCLE=1)
@@ -1049,7 +1082,17 @@ struct Gmres : SolverBase {
         CK(st.alloc(1));
         CK(cudaMemset(st.p, 0, sizeof(DevStatus)));
         const bool need_copy = (precond == VFV_PRECOND_JACOBI) || !std::is_same<T, double>::value;
-        if (need_copy) CK(valK.alloc(p->nnz));
+        if (engine != VFV_ENGINE_PERSISTENT && !p->sell_built) {
+            const int rc = build_pattern_sell(ctx, p);
+            if (rc) return rc;
+        }
+        sell = engine != VFV_ENGINE_PERSISTENT && p->sell_use;
+        if (sell) {
+            CK(valK.alloc(std::max<int64_t>(p->sell.slots, 1)));
+            CK(cudaMemsetAsync(valK.p, 0, valK.n * sizeof(T), ctx->stream));  // padding
+        } else if (need_copy) {
+            CK(valK.alloc(p->nnz));
+        }
         K.n = n;
         K.ldv = ldv;
         K.m = m;
@@ -1233,6 +1276,24 @@ struct Gmres : SolverBase {
         });
     }
 
+    // y = A x / beta_j with the Krylov matrix (SpMV of Arnoldi step j)
+    void enqueue_spmv(cudaStream_t s, vfv_pattern* p, const T* in, T* out, int j, bool pdl) {
+        const int lanes = p->spmv_lanes[sizeof(T) == 8 ? 0 : 1], strides = p->spmv_strides[sizeof(T) == 8 ? 0 : 1];
+        const T* vk = krylov_vals(p);
+        if (sell) {
+            const SellSeg seg{m + 1, j, nm, b_mesh_row.p};
+            const int64_t grid = grid_for(n, kSellWindow);
+            if (nm > 0)
+                launch_k(s, k_spmv_sell<T, true>, grid, kSellWindow, pdl, n, p->sell.dev(), p->sell_ci.p, vk, in, out, b_inv_beta.p, seg, st.p);
+            else
+                launch_k(s, k_spmv_sell<T, false>, grid, kSellWindow, pdl, n, p->sell.dev(), p->sell_ci.p, vk, in, out, inv_beta.p + j, seg, st.p);
+        } else if (nm > 0) {
+            launch_spmv_seg<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, out, b_inv_beta.p, m + 1, j, b_mesh_row.p, nm, st.p, pdl);
+        } else {
+            launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, out, inv_beta.p + j, st.p, pdl);
+        }
+    }
+
     // phase timestamps of the last cycle, averaged over its steps (diagnostics, VFV_TRACE_CYCLE=1)
     void dump_trace(vfv_ctx* ctx, int cycles) {
         std::vector<unsigned long long> h((size_t)(m + 2) * 8);
@@ -1276,7 +1337,7 @@ struct Gmres : SolverBase {
             in = z.p;
         }
         cudaEventRecord(ev[1], s);
-        launch_spmv<T, T, T, T>(s, p->spmv_lanes[sizeof(T) == 8 ? 0 : 1], p->spmv_strides[sizeof(T) == 8 ? 0 : 1], n, p->rp.p, p->ci.p, vk, in, w, inv_beta.p + j, st.p);
+        enqueue_spmv(s, p, in, w, j, false);
         cudaEventRecord(ev[2], s);
         enqueue_ortho(s, w, w, j);
         cudaEventRecord(ev[3], s);
@@ -1343,8 +1404,6 @@ struct Gmres : SolverBase {
     }
 
     void enqueue_step(cudaStream_t s, vfv_pattern* p, int j) {
-        const T* vk = krylov_vals(p);
-        const int lanes = p->spmv_lanes[sizeof(T) == 8 ? 0 : 1], strides = p->spmv_strides[sizeof(T) == 8 ? 0 : 1];
         T* w = V.p + (int64_t)(j + 1) * ldv;
         if (nm > 0) {  // one recurrence per mesh of a batch
             const T* uj = V.p + (int64_t)j * ldv;
@@ -1353,7 +1412,7 @@ struct Gmres : SolverBase {
                 apply_ilu(s, uj, z.p, st.p);
                 in = z.p;
             }
-            launch_spmv_seg<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, w, b_inv_beta.p, m + 1, j, b_mesh_row.p, nm, st.p, true);
+            enqueue_spmv(s, p, in, w, j, true);
             const int nv = j + 1, fb = grid_for((int64_t)nm * nv * 32);
             const bool pdl = shape == VecShape::small;  // as in enqueue_ortho
             with_shape(shape, [&](auto sh) {
@@ -1367,7 +1426,7 @@ struct Gmres : SolverBase {
             return;
         }
         if (engine == VFV_ENGINE_OVERLAP) {
-            launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, Zb.p + (int64_t)j * ldv, abuf.p, inv_beta.p + j, st.p, true);
+            enqueue_spmv(s, p, Zb.p + (int64_t)j * ldv, abuf.p, j, true);
             cudaEventRecord(ev_fork, s);
             cudaStreamWaitEvent(s2, ev_fork, 0);
             apply_ilu(s2, abuf.p, qbuf.p, st.p, ilu_prio, true);
@@ -1388,7 +1447,7 @@ struct Gmres : SolverBase {
             launch_k(s, k_bj4_apply<T>, grid_for(n / 4), 256, true, n / 4, bj_vals(), uj, z.p, st.p);
             in = z.p;
         }
-        launch_spmv<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, w, inv_beta.p + j, st.p, true);
+        enqueue_spmv(s, p, in, w, j, true);
         enqueue_ortho(s, w, w, j);
     }
 
@@ -1594,6 +1653,12 @@ struct Gmres : SolverBase {
         // matrix preparation for this solve
         if (valK.p && valk_version == p->version) {
             // the Krylov copy of the values is of this matrix already (time steps, adjoint solves)
+        } else if (sell) {
+            const bool jacobi = precond == VFV_PRECOND_JACOBI;
+            if (jacobi) k_jacobi_inv<<<grid_for(n), 256, 0, s>>>(n, p->diag_pos.p, p->val.p, dinv.p);
+            k_sell_vals<T><<<grid_for(n, kSellWindow), kSellWindow, 0, s>>>(n, p->sell.dev(), p->rp.p, p->ci.p, p->val.p,
+                                                                            jacobi ? dinv.p : nullptr, valK.p);
+            ctx->launches += jacobi ? 2 : 1;
         } else if (precond == VFV_PRECOND_JACOBI) {
             k_jacobi_inv<<<grid_for(n), 256, 0, s>>>(n, p->diag_pos.p, p->val.p, dinv.p);
             k_scale_cols<T><<<grid_for(p->nnz), 256, 0, s>>>(p->nnz, p->ci.p, p->val.p, dinv.p, valK.p);

@@ -211,6 +211,10 @@ struct vfv_pattern {
     DBuf<double> val;
     DBuf<float> val32;
     uint64_t version = 0, version32 = ~0ull;
+    // sliced rows of the solvers' SpMV (built by the first solver; not used when some row is long)
+    bool sell_built = false, sell_use = false;
+    SellBuf sell;
+    DBuf<int32_t> sell_ci;  // columns, -1: padding
     DBuf<int64_t> slot_ptr, slot_trip;
     DBuf<double> trip_vals;
     std::vector<int64_t> blocks;          // row ranges of the diagonal blocks of a block-diagonal system (may be empty)

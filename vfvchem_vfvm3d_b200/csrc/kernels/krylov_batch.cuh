@@ -61,16 +61,6 @@ struct BatchDev {
     const double* scal;        // [1]: mixed precision, a mesh's cycle also ends at resid_est <= scal[1] * beta0
 };
 
-__device__ __forceinline__ int mesh_of_row(const int64_t* __restrict__ mesh_row, int nm, int64_t row) {
-    int lo = 0, hi = nm;  // mesh_row[lo] <= row < mesh_row[hi]
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(mesh_row + mid) <= row) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // y = (A x) * inv_beta[mesh(row)][j]: the single-system SpMV with the step's scale looked up per row.
 template <typename TV, typename TX, typename TY, typename TA, int G, int S = 4>
 __global__ void __launch_bounds__(kBlk) k_spmv_seg(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
