@@ -154,9 +154,11 @@ struct IluStruct {
     DBuf<int> bad;
     uint64_t version64 = ~0ull, version32 = ~0ull;
 
-    // dataflow factorisation (k_ilu0_factor_flow): per-row ready flags holding the epoch of the
-    // factorisation that finished the row, the abort word and timeout flag of its bounded waits, and
+    // dataflow factorisation: short_rows, every row fits a warp's staging (k_ilu0_factor_flow); otherwise
+    // (k_ilu0_factor_flags) per-row ready flags holding the epoch of the factorisation that finished
+    // the row; the abort word and timeout flag of its bounded waits, and
     // the cooperative grid (0: not set up)
+    bool short_rows = false;
     DBuf<unsigned> ready, flow_state;
     unsigned epoch = 0;
     int flow_grid = 0;

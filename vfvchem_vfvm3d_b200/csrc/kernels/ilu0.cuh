@@ -87,7 +87,7 @@ __device__ __forceinline__ unsigned long long flow_clock_ns() {
     return t;
 }
 
-// Row readiness of the dataflow factorisation (k_ilu0_factor_flow): ready[k] == epoch once row k is
+// Row readiness of the dataflow factorisation by flags (k_ilu0_factor_flags): ready[k] == epoch once row k is
 // final. Waits poll with relaxed loads (one fence after the last one, by the caller); a wait gives up
 // after poll_limit polls or 2 s, raising *abort (which every waiting warp checks) and *timeout_flag.
 struct FlowSync {
@@ -139,6 +139,53 @@ struct FlowSync {
     }
 };
 
+// Structure of a row for a warp, lane l on entry l (column c): the pivot rows (one per lower entry t),
+// and where pivot row t's upper part has this lane's column, found by bisection (byte t of at: the
+// place, kFacNone: nowhere). False when the row, its lower entries or a pivot row are longer than the
+// staging.
+constexpr unsigned kFacNone = 0xffu;
+struct FacMatch {
+    unsigned at[kFacLow / 4];
+    __device__ __forceinline__ unsigned place(int t) const { return (at[t >> 2] >> (8 * (t & 3))) & 0xffu; }
+    __device__ __forceinline__ bool hit(int t) const { return place(t) != kFacNone; }
+};
+__device__ __forceinline__ bool factor_row_match(int32_t c, int32_t len, int32_t nl, const int32_t* __restrict__ rp,
+                                                 const int32_t* __restrict__ ci, const int32_t* __restrict__ dg, FacStage& sg,
+                                                 FacMatch& m) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    bool ok = len <= 32 && nl <= kFacLow;
+    if (ok && lane < nl) {
+        const int32_t dk = dg[c], ul = rp[c + 1] - dk - 1;
+        sg.k[lane] = c;
+        sg.dk[lane] = dk;
+        sg.len[lane] = ul;
+        if (ul > kFacUp) ok = false;
+    }
+    ok = __all_sync(full, ok);
+#pragma unroll
+    for (int q = 0; q < kFacLow / 4; ++q) m.at[q] = 0xffffffffu;
+    if (!ok) return false;
+    __syncwarp(full);
+    for (int idx = lane; idx < nl * kFacUp; idx += 32) {
+        const int t = idx / kFacUp, u = idx - t * kFacUp;
+        if (u < sg.len[t]) sg.col[t][u] = ci[sg.dk[t] + 1 + u];
+    }
+    __syncwarp(full);
+#pragma unroll
+    for (int t = 0; t < kFacLow; ++t) {
+        if (t < nl) {
+            const int ul = sg.len[t];
+            int u = 0;  // columns of the pivot row below c
+#pragma unroll
+            for (int st = 16; st > 0; st >>= 1)
+                if (u + st <= ul && sg.col[t][u + st - 1] < c) u += st;
+            if (lane > t && lane < len && u < ul && sg.col[t][u] == c) m.at[t >> 2] ^= (kFacNone ^ (unsigned)u) << (8 * (t & 3));
+        }
+    }
+    return true;
+}
+
 // Factors row i (one warp). FLOW: lane t waits for pivot row t through fs (values then read from
 // L2, past the SM's L1), and the row is published in ready[] when done; otherwise the previous level
 // has finished (programmatic dependent launch). False when a wait gave up.
@@ -151,43 +198,11 @@ __device__ __forceinline__ bool factor_row_warp(int32_t i, const int32_t* __rest
     auto piv_ld = [](const double* p) { return FLOW ? __ldcg(p) : *p; };
     const int32_t b = rp[i], e = rp[i + 1], d = dg[i];
     const int32_t len = e - b, nl = d - b;
-    bool ok = len <= 32 && nl <= kFacLow;
-    if (ok && lane < nl) {
-        const int32_t k = ci[b + lane];
-        const int32_t dk = dg[k], ul = rp[k + 1] - dk - 1;
-        sg.k[lane] = k;
-        sg.dk[lane] = dk;
-        sg.len[lane] = ul;
-        if (ul > kFacUp) ok = false;
-    }
-    ok = __all_sync(full, ok);
-    const int32_t c = ok && lane < len ? ci[b + lane] : -1;
+    // found before the wait; the eliminations after it are then one division and at most one
+    // multiply-subtract per pivot
+    FacMatch m;
+    const bool ok = factor_row_match(lane < len ? ci[b + lane] : -1, len, nl, rp, ci, dg, sg, m);
     double v = ok && lane < len ? a[b + lane] : 0.0;
-    // slot[t]: the slot of pivot row t's entry in this lane's column (-1: none). Structure only, so
-    // it is found before the wait; the eliminations after it are then one division and at most one
-    // multiply-subtract per pivot.
-    int32_t slot[kFacLow];
-#pragma unroll
-    for (int t = 0; t < kFacLow; ++t) slot[t] = -1;
-    if (ok) {
-        __syncwarp(full);
-        for (int idx = lane; idx < nl * kFacUp; idx += 32) {
-            const int t = idx / kFacUp, u = idx - t * kFacUp;
-            if (u < sg.len[t]) sg.col[t][u] = ci[sg.dk[t] + 1 + u];
-        }
-        __syncwarp(full);
-#pragma unroll
-        for (int t = 0; t < kFacLow; ++t) {
-            if (t < nl && lane > t && lane < len) {
-                const int ul = sg.len[t];
-                for (int u = 0; u < ul; ++u)
-                    if (sg.col[t][u] == c) {
-                        slot[t] = sg.dk[t] + 1 + u;
-                        break;
-                    }
-            }
-        }
-    }
     if constexpr (FLOW) {
         // lane t waits for pivot row t; all pivot loads come after every waiting lane's fence
         const bool has = ok && lane < nl;
@@ -240,7 +255,7 @@ __device__ __forceinline__ bool factor_row_warp(int32_t i, const int32_t* __rest
         const double ukk = lane < nl ? piv_ld(a + sg.dk[lane]) : 1.0;
         double mv[kFacLow];
 #pragma unroll
-        for (int t = 0; t < kFacLow; ++t) mv[t] = slot[t] >= 0 ? piv_ld(a + slot[t]) : 0.0;
+        for (int t = 0; t < kFacLow; ++t) mv[t] = m.hit(t) ? piv_ld(a + sg.dk[t] + 1 + m.place(t)) : 0.0;
         const bool zero = __any_sync(full, lane < nl && ukk == 0.0);
         if (!zero) {
 #pragma unroll
@@ -248,7 +263,7 @@ __device__ __forceinline__ bool factor_row_warp(int32_t i, const int32_t* __rest
                 if (t < nl) {
                     const double lik = __shfl_sync(full, v, t) / __shfl_sync(full, ukk, t);
                     if (lane == t) v = lik;
-                    if (slot[t] >= 0) v -= lik * mv[t];
+                    if (m.hit(t)) v -= lik * mv[t];
                 }
             }
         }
@@ -283,18 +298,121 @@ __global__ void __launch_bounds__(32 * kFacWarps) k_ilu0_factor_level_warp(int32
 // 692 levels on the 10^6-row heat matrix, ~12 us each as separate launches). Rows are in the
 // permuted numbering, where every pivot row of row i has a smaller index. Warp g of the W warps of
 // the grid factors rows g, g + W, g + 2W, ... in increasing order and, instead of waiting for a whole
-// level, waits only for its row's pivot rows (ready[k] == epoch). Progress needs every warp
-// resident (the smallest unfinished row always has all its pivots finished, and its warp has
-// finished all its earlier rows), hence a cooperative launch. Each row's arithmetic is
-// factor_row_warp's, so the factor is bit-identical to the level-by-level one.
-__global__ void __launch_bounds__(32 * kFacWarps) k_ilu0_factor_flow(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                                                     const int32_t* __restrict__ dg, double* a, int* __restrict__ bad,
-                                                                     FlowSync fs) {
+// level, waits only for its row's pivot rows. Progress needs every warp resident (the smallest
+// unfinished row always has all its pivots finished, and its warp has finished all its earlier rows),
+// hence a cooperative launch. Each row's arithmetic is factor_row_warp's, so the factor is
+// bit-identical to the level-by-level one.
+//
+// k_ilu0_factor_flow hands values over as their own flags: the factor starts as kFacOpen (all bits set,
+// a NaN that no row stores), A's values are read through src, and a row polls the very pivots and
+// entries that it needs with relaxed 64-bit loads. A hop of the chain is then a store, a load and one
+// elimination: no fences, no loads behind a flag, and pivots that are there already (the earlier
+// levels: the lower entries are sorted by level) are eliminated while the last ones are waited for.
+// Flags and fences -> values: 103,823 rows (319 levels) 1.37 -> 0.71 ms, 10^6 rows (692 levels)
+// 4.10 -> 2.77 ms: 2.2 us a level where few rows are in flight; at 10^6 the rows' own work (10 us for
+// the structure, the polls and the eliminations of a row, on 3,552 warps) bounds it. Four blocks per
+// SM (64 registers, spills) take 3.4 ms, two (125 registers, no prefetch) 4.05. k_ilu0_factor_flags (ready[k] == epoch once row k is
+// final) takes patterns with rows beyond the staging, whose serial rows work in place.
+__global__ void __launch_bounds__(32 * kFacWarps) k_ilu0_factor_flags(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                                                      const int32_t* __restrict__ dg, double* a, int* __restrict__ bad,
+                                                                      FlowSync fs) {
     __shared__ FacStage s_stage[kFacWarps];
     const int w = threadIdx.x >> 5;
     const int32_t nw = (int32_t)gridDim.x * kFacWarps;
     for (int32_t i = (int32_t)blockIdx.x * kFacWarps + w; i < n; i += nw)
         if (!factor_row_warp<true>(i, rp, ci, dg, a, bad, s_stage[w], fs)) return;
+}
+
+constexpr long long kFacOpen = -1ll;  // an entry of the factor that is not final yet
+__device__ __forceinline__ double ld_relaxed_gpu_f64(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool fac_open(double v) { return __double_as_longlong(v) == kFacOpen; }
+
+__global__ void __launch_bounds__(32 * kFacWarps, 3) k_ilu0_factor_flow(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                                                     const int32_t* __restrict__ dg, const int32_t* __restrict__ src,
+                                                                     const double* __restrict__ val, double* a, int* __restrict__ bad,
+                                                                     FlowSync fs) {
+    __shared__ FacStage s_stage[kFacWarps];
+    const unsigned full = 0xffffffffu;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    FacStage& sg = s_stage[w];
+    const int32_t nw = (int32_t)gridDim.x * kFacWarps;
+    // the next row's columns and sources, and the extent of the one after it, are on their way while a
+    // row is matched and waited for
+    struct Extent {
+        int32_t b, len, nl;
+    };
+    auto extent = [&](int64_t i) {
+        if (i >= n) return Extent{0, 0, 0};
+        const int32_t b = rp[i];
+        return Extent{b, rp[i + 1] - b, dg[i] - b};
+    };
+    const int64_t i0 = (int64_t)blockIdx.x * kFacWarps + w;
+    Extent r = extent(i0), r1 = extent(i0 + nw);
+    int32_t c1 = lane < r.len ? ci[r.b + lane] : -1, s1 = lane < r.len ? src[r.b + lane] : 0;
+    for (int64_t i = i0; i < n; i += nw) {
+        const int32_t b = r.b, len = r.len, nl = r.nl, c = c1;
+        const double v0 = lane < len ? val[s1] : 0.0;
+        __syncwarp(full);  // the last row's staging has been read
+        r = r1;
+        r1 = extent(i + 2 * (int64_t)nw);
+        c1 = lane < r.len ? ci[r.b + lane] : -1;
+        s1 = lane < r.len ? src[r.b + lane] : 0;
+        FacMatch m;
+        factor_row_match(c, len, nl, rp, ci, dg, sg, m);  // every row fits (IluStruct::short_rows)
+        double v = v0, ukk = lane < nl ? __longlong_as_double(kFacOpen) : 1.0;
+        const int32_t dk = lane < nl ? sg.dk[lane] : 0;
+        double mv[kFacLow];
+#pragma unroll
+        for (int t = 0; t < kFacLow; ++t) mv[t] = m.hit(t) ? __longlong_as_double(kFacOpen) : 0.0;
+        int done = 0;  // pivots eliminated, in the serial IKJ order
+        bool zero = false;
+        unsigned long long t0 = 0;
+        for (long long it = 0; done < nl; ++it) {
+            if (it > 0) {  // bounded: poll limit or 2 s
+                if (it == 1) t0 = flow_clock_ns();
+                int give_up = 0;
+                if (lane == 0) {
+                    if ((it & 15) == 0 && *(volatile unsigned*)fs.abort) give_up = 1;
+                    else if (it >= fs.poll_limit || ((it & 255) == 0 && flow_clock_ns() - t0 > 2000000000ull)) {
+                        atomicExch(fs.abort, 1u);
+                        *(volatile int*)fs.timeout_flag = 1;
+                        give_up = 1;
+                    }
+                }
+                if (__shfl_sync(full, give_up, 0)) return;
+                if (it > 8) __nanosleep(32);
+            }
+            if (fac_open(ukk)) ukk = ld_relaxed_gpu_f64(a + dk);
+#pragma unroll
+            for (int t = 0; t < kFacLow; ++t)
+                if (fac_open(mv[t])) mv[t] = ld_relaxed_gpu_f64(a + sg.dk[t] + 1 + m.place(t));
+#pragma unroll
+            for (int t = 0; t < kFacLow; ++t) {
+                if (t == done && t < nl && __all_sync(full, !fac_open(mv[t]) && !(lane == t && fac_open(ukk)))) {
+                    const double u = __shfl_sync(full, ukk, t);
+                    if (u == 0.0) zero = true;
+                    const double lik = __shfl_sync(full, v, t) / u;
+                    if (lane == t) v = lik;
+                    if (m.hit(t)) v -= lik * mv[t];
+                    done = t + 1;
+                }
+            }
+        }
+        if (zero) {  // reported; the row stays A's
+            if (lane == 0) *bad = 1;
+            v = v0;
+        } else if (lane == nl && v == 0.0) {
+            *bad = 1;
+        }
+        if (lane < len) {
+            if (fac_open(v)) v = __longlong_as_double(0x7fffffffffffffffll);
+            asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(a + b + lane), "d"(v) : "memory");
+        }
+    }
 }
 
 // Gather A's values into the permuted factor storage: lu[k] = (T) val[src[k]].
