@@ -278,9 +278,9 @@ def extras_transport(ctx, count):
 # roofline's traffic only when the bench runs that same matrix and lane count.
 SPMV_TRAFFIC_N100_4LANES = 209.2e6
 # DRAM bytes (read + write) of one k_ilu0_sweep<float, half values> launch on the same matrix (4-sweep
-# natural-order factors, 32-bit columns), from one ncu capture of a lower and an upper sweep
+# natural-order factors, 32-bit columns), averaged over the 8 sweeps of an apply, from one ncu capture
 # (profiles/k_ilu0_sweep_1M.md)
-SWEEP_TRAFFIC_N100 = 66.1e6
+SWEEP_TRAFFIC_N100 = 63.8e6
 
 
 def peaks():
@@ -508,8 +508,8 @@ def main():
 
     # The mixed solve's preconditioner timed alone: ILU_SWEEPS Jacobi sweeps of each factor in float
     # arithmetic over the row-scaled half-precision values (natural-order ILU(0) in A's numbering;
-    # 2 x ILU_SWEEPS k_ilu0_sweep launches per apply). Algorithmic bytes per sweep: the triangle's
-    # row pointer (4 (n+1)) and row scales (4 n), column indices (2 or 4 bytes) and half values (2)
+    # 2 x ILU_SWEEPS k_ilu0_sweep launches per apply). Algorithmic bytes per sweep: the slice offsets
+    # (4 per 32 rows), the position's row (1 byte) and row scales (4 n), column indices (2 or 4 bytes) and half values (2)
     # of its entries (nl = nu = (nnz - n) / 2 strictly lower / upper entries), right-hand side,
     # previous iterate and new iterate (12 n), the diagonal for the upper sweeps (4 n); the last
     # lower sweep also writes D^-1 u (4 n) and reads the diagonal (4 n).
@@ -520,7 +520,7 @@ def main():
     col_bytes = pat.ilu0_sweep_layout(L.ILU_NATURAL)
     ilu_launches = 2 * ILU_SWEEPS
     ntri = (nnz - n) // 2
-    bytes_ilu32 = ILU_SWEEPS * (2 * 4 * (n + 1) + (col_bytes + 2) * 2 * ntri + 36 * n) + 8 * n
+    bytes_ilu32 = ILU_SWEEPS * (2 * (n + n / 8) + (col_bytes + 2) * 2 * ntri + 36 * n) + 8 * n
     gbs_ilu32 = bytes_ilu32 / ilu_s / 1e9
     # the exact level-scheduled float apply (the FP64 baseline's preconditioner structure), for context
     ilu_nlev = pat.ilu0_apply_device_f32(rs32.data_ptr(), ts32.data_ptr(), zs32.data_ptr())
