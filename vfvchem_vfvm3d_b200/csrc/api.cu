@@ -140,12 +140,15 @@ void launch_spmv(cudaStream_t s, int lanes, int strides, int64_t n, const int32_
     switch (lanes * 16 + strides) {
 #define VFV_SHAPE_CASE(G, S)                                                                                               \
     case G * 16 + S:                                                                                                       \
-        launch_k(s, k_spmv<TV, TX, TY, TA, G, S>, grid_for(n * G), kBlk, pdl, n, rp, ci, val, x, y, scale, st);             \
+        if (st)                                                                                                            \
+            launch_k(s, k_spmv<TV, TX, TY, TA, G, S, true>, grid_for(n * G), kBlk, pdl, n, rp, ci, val, x, y, scale, st);   \
+        else                                                                                                               \
+            launch_k(s, k_spmv<TV, TX, TY, TA, G, S, false>, grid_for(n * G), kBlk, pdl, n, rp, ci, val, x, y, scale, st);  \
         return;
         VFV_SPMV_SHAPES(VFV_SHAPE_CASE)
 #undef VFV_SHAPE_CASE
         default:
-            launch_k(s, k_spmv<TV, TX, TY, TA, 4, 4>, grid_for(n * 4), kBlk, pdl, n, rp, ci, val, x, y, scale, st);
+            launch_spmv<TV, TX, TY, TA>(s, 4, 4, n, rp, ci, val, x, y, scale, st, pdl);
     }
 }
 

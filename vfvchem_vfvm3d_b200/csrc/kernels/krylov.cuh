@@ -127,14 +127,19 @@ __device__ __forceinline__ void row_load(RowFrag<TV, S>& f, const int32_t* __res
 }
 
 // x may have been written by the previous kernel of a programmatic-dependent-launch chain: plain loads
-template <typename TV, typename TX, typename TA, int G, int S>
+// unless RO
+template <typename TV, typename TX, typename TA, int G, int S, bool RO = false>
 __device__ __forceinline__ TA row_gather(const RowFrag<TV, S>& f, const int32_t* __restrict__ ci, const TV* __restrict__ val, const TX* x,
                                          int lane) {
     TA s = TA(0);
 #pragma unroll
     for (int t = 0; t < S; ++t)
-        if (f.c[t] >= 0) s += (TA)f.v[t] * (TA)x[f.c[t]];
-    for (int32_t k = f.b + lane + S * G; k < f.e; k += G) s += (TA)__ldcs(val + k) * (TA)x[__ldcs(ci + k)];
+        if (f.c[t] >= 0) s += (TA)f.v[t] * (TA)(RO ? __ldg(x + f.c[t]) : x[f.c[t]]);
+    for (int32_t k = f.b + lane + S * G; k < f.e; k += G) {
+        const TV v = __ldcs(val + k);
+        const int32_t c = __ldcs(ci + k);
+        s += (TA)v * (TA)(RO ? __ldg(x + c) : x[c]);
+    }
     return s;
 }
 
@@ -146,22 +151,25 @@ __device__ __forceinline__ TA row_dot(const int32_t* __restrict__ rp, const int3
     return row_gather<TV, TX, TA, G, S>(f, ci, val, x, lane);
 }
 
-// y = scale * (A x). Accumulation in TA. `scale` may be null (= 1). Inside a cycle graph the row's
-// indices and values, which no kernel of the cycle writes, are loaded before the wait for the
-// kernel that produces x.
-template <typename TV, typename TX, typename TY, typename TA, int G, int S = 4>
+// y = scale * (A x). Accumulation in TA. `scale` may be null (= 1). Inside a cycle graph (CHAIN) the
+// row's indices and values, which no kernel of the cycle writes, are loaded before the wait for the
+// kernel that produces x. Alone (st null) there is nothing to wait for and x may come through the
+// read-only path (4 lanes x 4: 262,144 rows double 16.3 -> 15.4 us, 10^6 rows float 36.9 -> 34.9).
+template <typename TV, typename TX, typename TY, typename TA, int G, int S, bool CHAIN>
 __global__ void __launch_bounds__(kBlk) k_spmv(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                               const TV* __restrict__ val, const TX* x, TY* y, const double* scale, const DevStatus* st) {
     const int lane = threadIdx.x & (G - 1);
     const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    const bool skip = st && st->done;  // set once and for all within a cycle: such a launch loads no rows
+    const bool skip = CHAIN && st->done;  // set once and for all within a cycle: such a launch loads no rows
     RowFrag<TV, S> f;
     if (row < n) row_load<TV, G, S>(f, rp, ci, val, row, lane, skip);
-    pdl_wait();
-    pdl_launch_dependents();
-    if (skip || (st && st->done)) return;
+    if constexpr (CHAIN) {
+        pdl_wait();
+        pdl_launch_dependents();
+        if (skip || st->done) return;
+    }
     TA s = TA(0);
-    if (row < n) s = row_gather<TV, TX, TA, G, S>(f, ci, val, x, lane);
+    if (row < n) s = row_gather<TV, TX, TA, G, S, !CHAIN>(f, ci, val, x, lane);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, G);
     if (lane == 0 && row < n) {
