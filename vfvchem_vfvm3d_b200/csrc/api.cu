@@ -975,6 +975,7 @@ struct Gmres : SolverBase {
     int nblk = 0, mega_grid = 0, mega_chunk = 0;
     VecShape shape = VecShape::wide;  // of the multi-vector kernels
     bool sell = false;                // valK and the SpMV in the pattern's sliced layout
+    int lanes = kSpG, strides = 4;    // SpMV shape, the pattern's when the solver was made: every cycle graph has the same
     DBuf<T> V, z, z2, zc, valK;
     DBuf<unsigned> bar;
     DBuf<unsigned long long> trace;  // per-phase timestamps of the last cycle (VFV_TRACE_CYCLE=1)
@@ -1041,6 +1042,8 @@ struct Gmres : SolverBase {
         ortho = ortho_;
         sweep_half = sweep_half_ && sweeps > 0 && !std::is_same<T, double>::value;
         ldv = (n + 63) / 64 * 64;
+        lanes = p->spmv_lanes[sizeof(T) == 8 ? 0 : 1];
+        strides = p->spmv_strides[sizeof(T) == 8 ? 0 : 1];
         shape = vec_shape<T>(n);
         nblk = (int)((n + shape_rows<T>(shape) - 1) / shape_rows<T>(shape));  // partial dots per vector
         const int64_t res_blocks = (n * kSpG + kBlk - 1) / kBlk;
@@ -1301,7 +1304,6 @@ struct Gmres : SolverBase {
 
     // y = A x / beta_j with the Krylov matrix (SpMV of Arnoldi step j)
     void enqueue_spmv(cudaStream_t s, vfv_pattern* p, const T* in, T* out, int j, bool pdl) {
-        const int lanes = p->spmv_lanes[sizeof(T) == 8 ? 0 : 1], strides = p->spmv_strides[sizeof(T) == 8 ? 0 : 1];
         const T* vk = krylov_vals(p);
         if (sell) {
             const SellSeg seg{m + 1, j, nm, b_mesh_row.p};
