@@ -152,13 +152,22 @@ int vfv_spmv_device(vfv_ctx* ctx, const vfv_pattern* p, const double* x, double*
 int vfv_spmv_device_f32(vfv_ctx* ctx, vfv_pattern* p, const float* x, float* y);
 /* Autotuner: measures the pattern's SpMV in each of its shapes (2 to 32 lanes per row, 1 to 8 strides
  * of indices and values loaded per lane before the gathers; double and float values) and keeps the
- * fastest for every later SpMV of this pattern and for solvers of patterns with long rows (solvers
- * keep short rows in slices of their own); call before its first solve. Returns the chosen lanes (either pointer may be NULL). */
+ * fastest for every later SpMV of this pattern and for the solvers that are made later; call before
+ * its first solve. Solvers of large patterns with short rows (189,440 rows and more, no row far longer
+ * than its neighbours) read them from slices of their own, a thread per row, and take from the shape
+ * the order in which the lanes sum a row; shapes of 16 and 32 lanes keep such solvers on CSR. Returns
+ * the chosen lanes (either pointer may be NULL). */
 int vfv_pattern_autotune(vfv_ctx* ctx, vfv_pattern* p, int32_t* lanes64, int32_t* lanes32);
-/* the SpMV shape in use: lanes per row and strides per lane, double and float (pointers may be NULL) */
+/* the SpMV shape of vfv_spmv_device(_f32) and of solvers made from now on (see vfv_pattern_autotune):
+ * lanes per row and strides per lane, double and float (pointers may be NULL) */
 int vfv_pattern_spmv_shape(const vfv_pattern* p, int32_t* lanes64, int32_t* strides64, int32_t* lanes32, int32_t* strides32);
-/* Sets the SpMV lanes per row by hand (2, 4, 8, 16 or 32 each, 4 strides per lane); VFV_BAD_INPUT otherwise. */
+/* Sets the SpMV lanes per row by hand (2, 4, 8, 16 or 32 each, 4 strides per lane); VFV_BAD_INPUT
+ * otherwise. Solvers that exist keep theirs; later ones sum their rows in the order of these lanes,
+ * whether they read them from CSR or from slices (see vfv_pattern_autotune). */
 int vfv_pattern_set_spmv_lanes(vfv_ctx* ctx, vfv_pattern* p, int32_t lanes64, int32_t lanes32);
+/* diagnostics: how many of the pattern's solvers read CSR rows and how many sliced rows, and the cycle
+ * graphs that they hold together (pointers may be NULL) */
+int vfv_pattern_solvers(const vfv_pattern* p, int32_t* csr, int32_t* sliced, int32_t* graphs);
 /* z = M^-1 r for the ILU(0) preconditioner of the pattern's current values (device arrays, double) */
 int vfv_ilu0_apply_device(vfv_ctx* ctx, vfv_pattern* p, int ilu_order, const double* r, double* z, int32_t* levels);
 /* z = M^-1 r with the float copy of the factor (the mixed-precision inner preconditioner), exposed

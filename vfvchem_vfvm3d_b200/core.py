@@ -239,13 +239,19 @@ class Pattern:
         return a.value, b.value
 
     def spmv_shape(self):
-        """((lanes, strides) double, (lanes, strides) float) of the SpMV in use."""
+        """((lanes, strides) double, (lanes, strides) float) of the SpMV and of solvers made from now on."""
         a, b, c, d = (C.c_int32() for _ in range(4))
         _check(self.ctx.handle, L.load().vfv_pattern_spmv_shape(self._h, C.byref(a), C.byref(b), C.byref(c), C.byref(d)))
         return (a.value, b.value), (c.value, d.value)
 
     def set_spmv_lanes(self, lanes64: int, lanes32: int) -> None:
         _check(self.ctx.handle, L.load().vfv_pattern_set_spmv_lanes(self.ctx.handle, self._h, int(lanes64), int(lanes32)))
+
+    def solvers(self):
+        """(solvers that read CSR rows, solvers that read sliced rows, their cycle graphs)"""
+        a, b, c = (C.c_int32() for _ in range(3))
+        _check(self.ctx.handle, L.load().vfv_pattern_solvers(self._h, C.byref(a), C.byref(b), C.byref(c)))
+        return a.value, b.value, c.value
 
     def ilu0_ordering(self, order: int = L.ILU_MULTICOLOR):
         """(perm new->old, lev_ptr) of the ILU(0) factor's symmetric permutation (host only)."""

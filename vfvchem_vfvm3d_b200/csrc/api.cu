@@ -940,6 +940,7 @@ constexpr int kFoldMax = 128;
 //    stays (residuals, factors), so a matrix that nearly fills the device is solved from CSR as it is.
 constexpr int64_t kSellRows = 148 * kSellBlocks * kSellWindow;
 constexpr int32_t kSellMost = 64;
+constexpr int kSellLanes = 8;  // widest CSR shape whose order of sums k_spmv_sell keeps (one register per lane)
 int build_pattern_sell(vfv_ctx* ctx, vfv_pattern* p) {
     p->sell_built = true;
     if (p->n < kSellRows) return VFV_OK;
@@ -1022,6 +1023,8 @@ struct Gmres : SolverBase {
     BatchDev B{};
     std::vector<MeshStat> mesh_stat;  // per-mesh state after the last solve
     long long wait_polls = kDefaultWaitPolls;  // bounded device waits of this solve (vfv_gmres_opts::wait_limit)
+    bool sliced() const override { return sell; }
+    int cycle_graphs() const override { return (int)graphs.size(); }
     ~Gmres() override {
         for (auto& g : graphs)
             if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
@@ -1108,11 +1111,14 @@ struct Gmres : SolverBase {
         CK(st.alloc(1));
         CK(cudaMemset(st.p, 0, sizeof(DevStatus)));
         const bool need_copy = (precond == VFV_PRECOND_JACOBI) || !std::is_same<T, double>::value;
-        if (engine != VFV_ENGINE_PERSISTENT && !p->sell_built) {
+        // lanes above kSellLanes: a shape for long rows, or one that the caller asked for
+        const char* rows_env = getenv("VFV_SOLVER_ROWS");  // diagnostics: "csr" keeps new solvers on CSR
+        const bool may_sell = engine != VFV_ENGINE_PERSISTENT && lanes <= kSellLanes && !(rows_env && std::string(rows_env) == "csr");
+        if (may_sell && !p->sell_built) {
             const int rc = build_pattern_sell(ctx, p);
             if (rc) return rc;
         }
-        sell = engine != VFV_ENGINE_PERSISTENT && p->sell_use;
+        sell = may_sell && p->sell_use;
         if (sell) {
             CK(valK.alloc(std::max<int64_t>(p->sell.slots, 1)));
             CK(cudaMemsetAsync(valK.p, 0, valK.n * sizeof(T), ctx->stream));  // padding
@@ -1307,11 +1313,21 @@ struct Gmres : SolverBase {
         const T* vk = krylov_vals(p);
         if (sell) {
             const SellSeg seg{m + 1, j, nm, b_mesh_row.p};
-            const int64_t grid = grid_for(n, kSellWindow);
-            if (nm > 0)
-                launch_k(s, k_spmv_sell<T, true>, grid, kSellWindow, pdl, n, p->sell.dev(), p->sell_ci.p, vk, in, out, b_inv_beta.p, seg, st.p);
-            else
-                launch_k(s, k_spmv_sell<T, false>, grid, kSellWindow, pdl, n, p->sell.dev(), p->sell_ci.p, vk, in, out, inv_beta.p + j, seg, st.p);
+            const double* scale = nm > 0 ? b_inv_beta.p : inv_beta.p + j;
+            switch (lanes * 2 + (nm > 0)) {
+#define VFV_SELL_CASE(G, SEG)                                                                                                        \
+    case G * 2 + SEG:                                                                                                                \
+        launch_k(s, k_spmv_sell<T, G, SEG != 0>, grid_for(n, kSellWindow), kSellWindow, pdl, n, p->sell.dev(), p->sell_ci.p, vk, in, \
+                 out, scale, seg, st.p);                                                                                             \
+        break;
+                VFV_SELL_CASE(2, 0)
+                VFV_SELL_CASE(2, 1)
+                VFV_SELL_CASE(4, 0)
+                VFV_SELL_CASE(4, 1)
+                VFV_SELL_CASE(8, 0)
+                VFV_SELL_CASE(8, 1)
+#undef VFV_SELL_CASE
+            }
         } else if (nm > 0) {
             launch_spmv_seg<T, T, T, T>(s, lanes, strides, n, p->rp.p, p->ci.p, vk, in, out, b_inv_beta.p, m + 1, j, b_mesh_row.p, nm, st.p, pdl);
         } else {
@@ -2397,8 +2413,9 @@ int vfv_ilu0_apply_device_noalloc(vfv_ctx* ctx, vfv_pattern* p, int ilu_order, c
 // Autotuner: times the SpMV of this pattern (its current values) in every shape of kSpmvShapes
 // (2 to 32 lanes per row, 1 to 8 strides loaded per lane before the gathers) in double and in float
 // (short rows of a scalar problem favour few lanes, the 2-ring rows of the coupled flow system a
-// warp per row), keeps the fastest of each for every later SpMV and solver of the pattern.
-// Must run before the pattern's first solve (solvers capture their kernels once).
+// warp per row), keeps the fastest of each for every later SpMV and for solvers made later. Solvers of
+// patterns in the sliced layout take over the order of sums of the lanes (up to kSellLanes), not the
+// strides. A solver keeps the shape that it was made with.
 int vfv_pattern_autotune(vfv_ctx* ctx, vfv_pattern* p, int32_t* lanes64, int32_t* lanes32) {
     DeviceGuard dg_(ctx);
     if (!ctx || !p) return set_err(ctx, VFV_BAD_INPUT, "NULL argument");
@@ -2470,6 +2487,19 @@ int vfv_pattern_set_spmv_lanes(vfv_ctx* ctx, vfv_pattern* p, int32_t lanes64, in
     p->spmv_lanes[0] = lanes64;
     p->spmv_lanes[1] = lanes32;
     p->spmv_strides[0] = p->spmv_strides[1] = 4;
+    return VFV_OK;
+}
+
+int vfv_pattern_solvers(const vfv_pattern* p, int32_t* csr, int32_t* sliced, int32_t* graphs) {
+    if (!p) return set_err(nullptr, VFV_BAD_INPUT, "pattern is NULL");
+    int32_t c = 0, l = 0, g = 0;
+    for (const auto& s : p->solvers) {
+        (s.second->sliced() ? l : c) += 1;
+        g += s.second->cycle_graphs();
+    }
+    if (csr) *csr = c;
+    if (sliced) *sliced = l;
+    if (graphs) *graphs = g;
     return VFV_OK;
 }
 

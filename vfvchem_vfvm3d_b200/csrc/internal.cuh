@@ -201,6 +201,8 @@ struct IluStruct {
 
 struct SolverBase {
     virtual ~SolverBase() = default;
+    virtual bool sliced() const = 0;       // its SpMV reads the pattern's sliced rows (CSR otherwise)
+    virtual int cycle_graphs() const = 0;  // cycle graphs that it holds
 };
 
 struct vfv_pattern {

@@ -200,11 +200,18 @@ __global__ void __launch_bounds__(kBlk) k_spmv(int64_t n, const int32_t* __restr
 
 // The solvers' SpMV of matrices with short rows: a thread per row of the sliced layout (SellDev), whose
 // indices and values a warp reads in full lines; several lanes per CSR row read runs of 16 to 32 bytes.
-// The first K entries are loaded before the wait for the kernel that produces x. Entries are summed in
-// column order. Alone on the 10^6-row heat matrix, CSR with the autotuned lanes and sliced: float
-// 33.1 -> 26.9 us, double 47.3 -> 38.8 us (5.5 TB/s of the matrix's bytes); 103,823 rows 8.3 -> 6.2
-// us. scale: the step's 1 / beta_j (SEG: looked up per row from its mesh, scale[mesh * stride + j]).
-constexpr int kSellBlocks = 5;  // resident blocks per SM of the double kernel (float: 8)
+// The first K entries are loaded before the wait for the kernel that produces x. The thread keeps one
+// sum per lane of the CSR shape (entry q of the row in sum q mod G) and adds them as the lanes' shuffles
+// do, so that a row's product has the same bits in either layout: which of them a solver reads can go by
+// the size of the whole system. Alone on the 10^6-row heat matrix with one sum per row, CSR with the
+// autotuned lanes and sliced: float 33.1 -> 26.9 us, double 47.3 -> 38.8 us (5.5 TB/s of the matrix's
+// bytes); 103,823 rows 8.3 -> 6.2 us. The lanes' sums cost nothing that whole solves show (10^6 rows mixed
+// 89.0 ms with one sum and with four, 262,144 rows FP64 32.6 / 32.7, a batch of 884,000 rows 33.9 / 34.3).
+// scale: the step's 1 / beta_j (SEG: looked up per row from its mesh, scale[mesh * stride + j]).
+constexpr int kSellBlocks = 5;  // resident blocks per SM of the double kernel
+// the float kernel's: full SMs while the lanes' sums fit 32 registers (with more sums it spills)
+template <typename T, int G, bool SEG>
+constexpr int kSellMinBlocks = sizeof(T) == 8 ? kSellBlocks : G == 8 ? 6 : G == 4 && SEG ? 7 : 8;
 struct SellSeg {
     int stride, j, nm;
     const int64_t* mesh_row;
@@ -219,11 +226,12 @@ __device__ __forceinline__ int mesh_of_row(const int64_t* __restrict__ mesh_row,
     return lo;
 }
 
-template <typename T, bool SEG>
-__global__ void __launch_bounds__(kSellWindow, sizeof(T) == 4 ? 8 : kSellBlocks)
+template <typename T, int G, bool SEG>
+__global__ void __launch_bounds__(kSellWindow, (kSellMinBlocks<T, G, SEG>))
     k_spmv_sell(int64_t n, SellDev S, const int32_t* __restrict__ ci, const T* __restrict__ val, const T* x, T* y, const double* scale, SellSeg seg,
                 const DevStatus* st) {
     constexpr int K = 8;
+    static_assert(K % G == 0, "entry q goes to sum q mod G");
     const int32_t t = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const bool skip = st && st->done;  // set once and for all within a cycle: such a launch loads no rows
     const int32_t k0 = __ldg(S.so + (t >> 5)), k1 = __ldg(S.so + (t >> 5) + 1);
@@ -241,10 +249,12 @@ __global__ void __launch_bounds__(kSellWindow, sizeof(T) == 4 ? 8 : kSellBlocks)
     pdl_wait();
     pdl_launch_dependents();
     if (skip || (st && st->done)) return;
-    T s = T(0);
+    T s[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) s[g] = T(0);
 #pragma unroll
     for (int q = 0; q < K; ++q)
-        if (c[q] >= 0) s += v[q] * x[c[q]];
+        if (c[q] >= 0) s[q % G] += v[q] * x[c[q]];
     for (int q0 = K; q0 < w; q0 += K) {
 #pragma unroll
         for (int q = 0; q < K; ++q) {
@@ -253,13 +263,18 @@ __global__ void __launch_bounds__(kSellWindow, sizeof(T) == 4 ? 8 : kSellBlocks)
         }
 #pragma unroll
         for (int q = 0; q < K; ++q)
-            if (c[q] >= 0) s += v[q] * x[c[q]];
+            if (c[q] >= 0) s[q % G] += v[q] * x[c[q]];
     }
-    if (row < n) y[row] = (T)((double)s * scale[SEG ? (int64_t)mesh * seg.stride + seg.j : 0]);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int g = 0; g < o; ++g) s[g] += s[g + o];
+    if (row < n) y[row] = (T)((double)s[0] * scale[SEG ? (int64_t)mesh * seg.stride + seg.j : 0]);
 }
 
 // out = (T)(val[k] * dinv[col[k]]) in the sliced layout (right Jacobi scaling folded into the Krylov
-// matrix; dinv null: the values), a thread per position; padding is left as it is
+// matrix; dinv null: the values), a thread per position; padding is left as it is. For layouts without
+// tails (build_pattern_sell keeps no others): every entry of a row lies within its slice's width.
 template <typename T>
 __global__ void __launch_bounds__(kSellWindow) k_sell_vals(int64_t n, SellDev S, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                                           const double* __restrict__ val, const double* __restrict__ dinv,
