@@ -907,6 +907,15 @@ void with_shape(VecShape v, F fn) {
     else fn(VecSmall{});
 }
 
+// fn(shape type, whether the update kernels fold)
+template <typename F>
+void with_shape_fold(VecShape v, bool fold, F fn) {
+    with_shape(v, [&](auto sh) {
+        if (fold) fn(sh, std::true_type{});
+        else fn(sh, std::false_type{});
+    });
+}
+
 template <typename T>
 int64_t shape_rows(VecShape v) {
     int64_t r = 0;
@@ -975,6 +984,7 @@ struct Gmres : SolverBase {
     int m = 0, precond = 0, ilu_order = 0, engine = 0;
     int nblk = 0, mega_grid = 0, mega_chunk = 0;
     VecShape shape = VecShape::wide;  // of the multi-vector kernels
+    bool fold = false;                // the update kernels sum the few partial dots themselves (no launch for them)
     bool sell = false;                // valK and the SpMV in the pattern's sliced layout
     int lanes = kSpG, strides = 4;    // SpMV shape, the pattern's when the solver was made: every cycle graph has the same
     DBuf<T> V, z, z2, zc, valK;
@@ -1129,7 +1139,7 @@ struct Gmres : SolverBase {
         K.ldv = ldv;
         K.m = m;
         K.nblk = nblk;
-        K.fold = nblk <= kFoldMax;
+        fold = nblk <= kFoldMax;
         K.part = part.p;
         K.counter = counter.p;
         K.hacc = hacc.p;
@@ -1224,7 +1234,7 @@ struct Gmres : SolverBase {
         CK(cudaMemset(b_counter.p, 0, 4 * sizeof(unsigned)));
         CK(b_mesh_counter.alloc(nm));
         B.mesh_counter = b_mesh_counter.p;
-        B.fold = most <= kFoldMax;
+        fold = most <= kFoldMax;
         B.nm = nm;
         B.m = m;
         B.ldv = ldv;
@@ -1283,28 +1293,29 @@ struct Gmres : SolverBase {
     // unless the first pass's test asked for it; VFV_ORTHO_CGS: the first pass alone.
     void enqueue_ortho(cudaStream_t s, const T* win, T* w, int j) {
         const int nv = j + 1, fb = grid_for((int64_t)nv * 32), fb1 = grid_for((int64_t)(nv + 1) * 32);
-        const bool cgs2 = ortho == VFV_ORTHO_CGS2, fold = K.fold != 0;
+        const bool cgs2 = ortho == VFV_ORTHO_CGS2;
         const int dgks = ortho == VFV_ORTHO_DGKS ? 1 : 0;
         const T* basis = V.p;
         // Programmatic dependent launch where the kernel or the one before it leaves most SMs free. A
         // grid of one or two blocks per SM that starts among the last blocks of the one before lands
         // unevenly on the SMs (FP64 solve of 125,000 rows 19.9 against 17.5 ms).
         const bool pdl = shape == VecShape::small;
-        with_shape(shape, [&](auto sh) {
+        with_shape_fold(shape, fold, [&](auto sh, auto folds) {
             using S = decltype(sh);
+            constexpr bool F = decltype(folds)::value && std::is_same<S, VecSmall>::value;  // kFoldMax blocks are fewer than VecMid's
             launch_k(s, k_mdot<T, S>, nblk, kBlk, false, K, basis, win, nv, dgks, 0);
-            if (!fold) launch_k(s, k_dots_finish<true>, dgks ? fb1 : fb, 256, true, K, nv, dgks, 0);
+            if (!F) launch_k(s, k_dots_finish<true>, dgks ? fb1 : fb, 256, true, K, nv, dgks, 0);
             if (cgs2) {
-                launch_k(s, k_update<T, S, false>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, 0, 0);
-                if (!fold) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 0);
-                launch_k(s, k_update<T, S, true>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 0);
+                launch_k(s, k_update<T, S, false, F>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, 0, 0);
+                if (!F) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 0);
+                launch_k(s, k_update<T, S, true, F>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 0);
                 return;
             }
-            launch_k(s, k_update<T, S, true>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, dgks, 0);
+            launch_k(s, k_update<T, S, true, F>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, dgks, 0);
             if (!dgks) return;
             launch_k(s, k_mdot<T, S>, nblk, kBlk, false, K, basis, w, nv, 0, 1);
-            if (!fold) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 1);
-            launch_k(s, k_update<T, S, true>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 1);
+            if (!F) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 1);
+            launch_k(s, k_update<T, S, true, F>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 1);
         });
     }
 
@@ -1456,13 +1467,14 @@ struct Gmres : SolverBase {
             enqueue_spmv(s, p, in, w, j, true);
             const int nv = j + 1, fb = grid_for((int64_t)nm * nv * 32);
             const bool pdl = shape == VecShape::small;  // as in enqueue_ortho
-            with_shape(shape, [&](auto sh) {
+            with_shape_fold(shape, fold, [&](auto sh, auto folds) {
                 using S = decltype(sh);
+                constexpr bool F = decltype(folds)::value;
                 launch_k(s, k_bmdot<T, S>, B.ntile, kBlk, false, B, V.p, w, nv);
-                if (!B.fold) launch_k(s, k_bdots_finish<true>, fb, 256, true, B, nv);
-                launch_k(s, k_bupdate<T, S, false>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
-                if (!B.fold) launch_k(s, k_bdots_finish<false>, fb, 256, true, B, nv);
-                launch_k(s, k_bupdate<T, S, true>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
+                if (!F) launch_k(s, k_bdots_finish<true>, fb, 256, true, B, nv);
+                launch_k(s, k_bupdate<T, S, false, F>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
+                if (!F) launch_k(s, k_bdots_finish<false>, fb, 256, true, B, nv);
+                launch_k(s, k_bupdate<T, S, true, F>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
             });
             return;
         }

@@ -51,7 +51,6 @@ struct KrylovDev {
     int64_t ldv;        // stride between basis vectors (elements)
     int m;              // restart length
     int nblk;           // blocks of the multi-vector kernels
-    int fold;           // the update kernels sum the partial dots themselves (few blocks; no k_dots_finish)
     double* part;       // [3][kMaxBasis][nblk] per-block partial dots: first pass, second pass, ||w||^2
     unsigned* counter;  // [4] last-block counters
     double* hacc;       // [kMaxBasis] current Hessenberg column (accumulated over the CGS passes)
@@ -462,8 +461,7 @@ __device__ __forceinline__ void sum_columns(const double* part, int64_t ld, int 
 }
 
 // ---------------------------------------------------------------- multi-dot (first CGS pass)
-// Per-block partials of d_i = <u_i, w> for i < nvec (summed by k_dots_finish<true>, or by the update
-// kernel when K.fold is set). with_norm: also the partials of ||w||^2, as vector nvec (the first pass
+// Per-block partials of d_i = <u_i, w> for i < nvec (summed by k_dots_finish<true>, or by k_update<FOLD>). with_norm: also the partials of ||w||^2, as vector nvec (the first pass
 // of the reorthogonalise-if-needed scheme); only_reorth: a second pass (its partials go to the second
 // buffer), skipped unless the first pass asked for it.
 template <typename T, class S>
@@ -595,9 +593,10 @@ __device__ __forceinline__ ColumnEnd arnoldi_column(const ColumnDst& D, ColumnSm
 // FINAL == true, ||w||^2 and the last block finishes the Hessenberg column j, the Givens rotation
 // and the convergence test - unless dgks is set and the test asks for a second pass, whose own
 // k_update (launched with only_reorth) then finishes the column. second: the coefficients come from
-// the second pass. With K.fold every block sums the (few) partials itself instead of reading the
-// coefficients that k_dots_finish left.
-template <typename T, class S, bool FINAL>
+// the second pass. FOLD: every block sums the (few) partials itself instead of reading the coefficients
+// that k_dots_finish left; a template argument, for the sums' registers would spill in the shapes of
+// many blocks, which never fold (VecWide, 32 registers, 10^6 rows).
+template <typename T, class S, bool FINAL, bool FOLD>
 __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_update(KrylovDev K, const T* V, const T* win, T* w, int nvec, int j, int second,
                                                                 int dgks, int only_reorth) {
     pdl_wait();
@@ -609,7 +608,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_update(KrylovDev K, con
     __shared__ double s_acc[S::kVS > 1 ? kBlk * R : 1];
     __shared__ ColumnSmem s_col;
     double* h = s_col.h;
-    if (K.fold) {
+    if constexpr (FOLD) {
         sum_columns(K.part + (second ? (int64_t)kMaxBasis * K.nblk : 0), K.nblk, K.nblk, nvec, [&](int c, double s) {
             const double ib = K.inv_beta[c], hc = s * ib, cf = hc * ib;
             s_coef[c] = cf;
@@ -667,7 +666,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_update(KrylovDev K, con
         double wn2 = 0.0;
         if (dgks) {
             __syncthreads();
-            wn2 = K.fold ? reduce_partials(K.part + (int64_t)nvec * K.nblk, K.nblk, red[0]) : K.wnorm2[0];
+            wn2 = FOLD ? reduce_partials(K.part + (int64_t)nvec * K.nblk, K.nblk, red[0]) : K.wnorm2[0];
         }
         if (threadIdx.x == 0) {
             K.counter[3] = 0u;

@@ -41,7 +41,6 @@ struct BatchDev {
     const int32_t* rtile_mesh; // [nrtile]
     const int32_t* mesh_rtile; // [nm+1]
     int ntile, nrtile;
-    int fold;                  // the update kernels sum the mesh's partial dots themselves (no k_bdots_finish)
     double* part;              // [3][kMaxBasis][ntile] per-tile partial dots: first pass, second pass, ||w||^2
     double* rpart;             // [2][nrtile] per-tile partial norms of the residual and of b
     double* hacc;              // [nm][kMaxBasis]
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__(256) k_bdots_finish(BatchDev B, int nvec) {
 // per-tile ||w||^2, and the mesh's last tile to arrive completes its Arnoldi step j: Hessenberg
 // column, Givens rotation, stopping test (k_update's arithmetic). The last mesh to stop sets the
 // global done flag.
-template <typename T, class S, bool FINAL>
+template <typename T, class S, bool FINAL, bool FOLD>
 __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, const T* V, const T* win, T* w, int nvec, int j) {
     pdl_wait();
     pdl_launch_dependents();
@@ -288,7 +287,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, con
     double* cs = B.cs + (int64_t)m * B.m;
     double* sn = B.sn + (int64_t)m * B.m;
     const double* inv_beta = B.inv_beta + (int64_t)m * m1;
-    if (B.fold) {
+    if constexpr (FOLD) {
         sum_columns(B.part + (FINAL ? (int64_t)kMaxBasis * B.ntile : 0) + t0, B.ntile, nt, nvec, [&](int c, double s) {
             const double ib = inv_beta[c], hc = s * ib;
             s_coef[c] = hc * ib;
