@@ -933,11 +933,6 @@ VecShape vec_shape(int64_t rows) {
     return blocks >= 800 ? VecShape::wide : blocks >= 150 ? VecShape::mid : VecShape::small;
 }
 
-// Up to this many partials per vector the update kernels sum them themselves: two launches per
-// Arnoldi step less (8,000 rows: 3.57 against 3.65 ms per solve; 400 partials already cost more than
-// the launches they save, 130 against 118 ms at 131,072 rows).
-constexpr int kFoldMax = 128;
-
 // The sliced rows of a pattern's SpMV: wanted
 //  - for a full wave of the sliced kernel's resident blocks, 148 x 5 x 256 rows: with fewer, a thread
 //    per row leaves the chip idle and several lanes per CSR row are faster (8,000 rows: 3.27 against
@@ -1183,8 +1178,8 @@ struct Gmres : SolverBase {
         return VFV_OK;
     }
 
-    // Tiles of the batched kernels from the mesh row ranges, inside one mesh each: vector tiles that
-    // start on 16-byte boundaries but for a mesh's first, and residual tiles of kBlk / kSpG rows.
+    // Tiles of the batched kernels from the mesh row ranges: vector tiles of a block's rows and residual
+    // tiles of kBlk / kSpG rows, each starting at its mesh's first row.
     int init_batch(vfv_ctx* ctx, const std::vector<int64_t>& rows) {
         nm = (int)rows.size() - 1;
         std::vector<int64_t> tr, rr;
@@ -1194,8 +1189,8 @@ struct Gmres : SolverBase {
         for (int q = 0; q < nm; ++q) {
             mt[q] = (int32_t)tm.size();
             mr[q] = (int32_t)rm.size();
-            for (int64_t r = rows[q] / kVecRows<T> * kVecRows<T>; r < rows[q + 1]; r += tv) {
-                tr.push_back(std::max(r, rows[q]));
+            for (int64_t r = rows[q]; r < rows[q + 1]; r += tv) {
+                tr.push_back(r);
                 tm.push_back(q);
             }
             most = std::max(most, (int)tm.size() - mt[q]);
@@ -1304,17 +1299,17 @@ struct Gmres : SolverBase {
             using S = decltype(sh);
             constexpr bool F = decltype(folds)::value && std::is_same<S, VecSmall>::value;  // kFoldMax blocks are fewer than VecMid's
             launch_k(s, k_mdot<T, S>, nblk, kBlk, false, K, basis, win, nv, dgks, 0);
-            if (!F) launch_k(s, k_dots_finish<true>, dgks ? fb1 : fb, 256, true, K, nv, dgks, 0);
+            if (!F) launch_k(s, k_dots_finish<S, true>, dgks ? fb1 : fb, 256, true, K, nv, dgks, 0);
             if (cgs2) {
                 launch_k(s, k_update<T, S, false, F>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, 0, 0);
-                if (!F) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 0);
+                if (!F) launch_k(s, k_dots_finish<S, false>, fb, 256, true, K, nv, 0, 0);
                 launch_k(s, k_update<T, S, true, F>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 0);
                 return;
             }
             launch_k(s, k_update<T, S, true, F>, nblk, kBlk, pdl, K, basis, win, w, nv, j, 0, dgks, 0);
             if (!dgks) return;
             launch_k(s, k_mdot<T, S>, nblk, kBlk, false, K, basis, w, nv, 0, 1);
-            if (!F) launch_k(s, k_dots_finish<false>, fb, 256, true, K, nv, 0, 1);
+            if (!F) launch_k(s, k_dots_finish<S, false>, fb, 256, true, K, nv, 0, 1);
             launch_k(s, k_update<T, S, true, F>, nblk, kBlk, pdl, K, basis, w, w, nv, j, 1, 0, 1);
         });
     }
@@ -1471,9 +1466,9 @@ struct Gmres : SolverBase {
                 using S = decltype(sh);
                 constexpr bool F = decltype(folds)::value;
                 launch_k(s, k_bmdot<T, S>, B.ntile, kBlk, false, B, V.p, w, nv);
-                if (!F) launch_k(s, k_bdots_finish<true>, fb, 256, true, B, nv);
+                if (!F) launch_k(s, k_bdots_finish<S, true>, fb, 256, true, B, nv);
                 launch_k(s, k_bupdate<T, S, false, F>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
-                if (!F) launch_k(s, k_bdots_finish<false>, fb, 256, true, B, nv);
+                if (!F) launch_k(s, k_bdots_finish<S, false>, fb, 256, true, B, nv);
                 launch_k(s, k_bupdate<T, S, true, F>, B.ntile, kBlk, pdl, B, V.p, w, w, nv, j);
             });
             return;

@@ -29,16 +29,21 @@ template <typename T>
 constexpr int kVecRows = 16 / (int)sizeof(T);
 
 // Shapes of the multi-vector kernels. A block's threads form kVS groups; every group owns the same
-// tile of rows and takes each kVS-th basis vector, loading the chunks of kGV of its vectors before
-// it uses any of them. kMinBlocks bounds the registers.
+// tile of rows and takes each kVS-th basis vector's dot, loading the chunks of kGV of its vectors
+// before it uses any of them. In an update the vectors form kChains chains; a thread adds up kCA of them
+// at a time (one of float rows: registers), loading the chunks of kGU vectors of each. kMinBlocks bounds the registers.
+// All shapes give the same bits, for the shape goes by the rows of a whole batch while a mesh's iterates
+// must not: a dot is summed over 64 chunks (two warps, one block of VecSmall), then over four such in
+// turn (one block of the others), then over those as in sum_groups; an update adds up the basis vectors
+// in the same kChains chains.
 struct VecWide {  // many rows: a full SM of threads hides the latency
-    static constexpr int kGV = 2, kVS = 1, kMinBlocks = 8;
+    static constexpr int kGV = 2, kGU = 2, kCA = 1, kVS = 1, kMinBlocks = 8, kPer = 1;
 };
 struct VecMid {  // a few blocks per SM: more loads in flight per thread instead
-    static constexpr int kGV = 8, kVS = 1, kMinBlocks = 4;
+    static constexpr int kGV = 8, kGU = 4, kCA = 2, kVS = 1, kMinBlocks = 4, kPer = 1;
 };
-struct VecSmall {  // fewer blocks than SMs: the basis is split over the block's warps as well
-    static constexpr int kGV = 8, kVS = 4, kMinBlocks = 3;
+struct VecSmall {  // fewer blocks than SMs: smaller tiles, and the basis is split over the block's warps as well
+    static constexpr int kGV = 8, kGU = 8, kCA = 1, kVS = 4, kMinBlocks = 3, kPer = 4;  // kPer: blocks whose partials are added first
 };
 template <typename T, class S>
 __host__ __device__ constexpr int64_t vec_block_rows() {
@@ -91,11 +96,46 @@ __device__ __forceinline__ void publish_partial(double* p, double v) {
     __threadfence();
 }
 
-// Sum column c of part[c][0..nblk) with all threads of the block, in a fixed order; valid in thread 0.
+// Sum of the q-th PER of the nb partials, in order
+template <int PER>
+__device__ __forceinline__ double partial_group(const double* part, int q, int nb) {
+    double v[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) v[u] = PER * q + u < nb ? __ldcg(part + PER * q + u) : 0.0;
+    double s = v[0];
+#pragma unroll
+    for (int u = 1; u < PER; ++u) s += v[u];
+    return s;
+}
+
+// Sum of part[0..nblk) with all threads of the block, PER partials first, in a fixed order; valid in thread 0.
+template <int PER = 1>
 __device__ __forceinline__ double reduce_partials(const double* part, int nblk, double* red) {
     double s = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += __ldcg(part + b);
+    for (int q = threadIdx.x; PER * q < nblk; q += blockDim.x) s += partial_group<PER>(part, q, nblk);
     return block_sum(s, red);
+}
+
+// Sum of part[0..nb) with one warp, PER partials first, in a fixed order; valid in every lane.
+template <int PER>
+__device__ __forceinline__ double sum_groups(const double* part, int nb) {
+    const int lane = threadIdx.x & 31, ng = (nb + PER - 1) / PER;
+    constexpr int kB = 16;
+    double s = 0.0;
+    for (int q0 = 0; q0 < ng; q0 += 32 * kB) {
+        double v[kB];
+#pragma unroll
+        for (int k = 0; k < kB; ++k) {
+            const int q = q0 + lane + 32 * k;
+            v[k] = q < ng ? partial_group<PER>(part, q, nb) : 0.0;
+        }
+#pragma unroll
+        for (int h = kB / 2; h > 0; h >>= 1)
+#pragma unroll
+            for (int k = 0; k < h; ++k) v[k] += v[k + h];
+        s += v[0];
+    }
+    return warp_sum(s);
 }
 
 // ---------------------------------------------------------------- SpMV (CSR, G lanes per row)
@@ -328,16 +368,16 @@ __global__ void __launch_bounds__(kBlk) k_residual(KrylovDev K, const int32_t* _
 }
 
 // ---------------------------------------------------------------- grouped multi-vector passes
-// A thread owns the kVecRows<T> consecutive rows of one 16-byte chunk, of which the rows [lo, hi) lie
-// in the tile; the others read as zero and are not written. A chunk is moved with one 16-byte load or
-// store when it is complete, else row by row. Chunks start on 16-byte boundaries, so a tile that
-// starts at any row (the batched kernels' per-mesh tiles) has ragged chunks at its two ends only. Per
-// vector the thread's rows are summed in row order, then across the warp (butterfly), the group's
-// warps and the blocks, in fixed orders.
+// A thread owns a chunk of kVecRows<T> consecutive rows, counted from its tile's first row, of which
+// `cnt` lie in the tile; the others read as zero and are not written. A complete chunk on a 16-byte
+// boundary is moved with one load or store, any other row by row: the last one of a tile, and all of a
+// tile that starts off such a boundary (the batched kernels' meshes at odd rows). Per vector the
+// thread's rows are summed in row order, then across the warp (butterfly), the block's warps and the
+// blocks, in fixed orders.
 template <typename T>
-__device__ __forceinline__ void load_chunk(const T* p, int lo, int hi, T (&x)[kVecRows<T>]) {
+__device__ __forceinline__ void load_chunk(const T* p, int cnt, bool aligned, T (&x)[kVecRows<T>]) {
     constexpr int R = kVecRows<T>;
-    if (hi - lo == R) {
+    if (cnt == R && aligned) {
         if constexpr (R == 4) {
             const float4 t = *reinterpret_cast<const float4*>(p);
             x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
@@ -347,39 +387,48 @@ __device__ __forceinline__ void load_chunk(const T* p, int lo, int hi, T (&x)[kV
         }
     } else {
 #pragma unroll
-        for (int r = 0; r < R; ++r) x[r] = r >= lo && r < hi ? p[r] : T(0);
+        for (int r = 0; r < R; ++r) x[r] = r < cnt ? p[r] : T(0);
     }
 }
 
 template <typename T>
-__device__ __forceinline__ void store_chunk(T* p, int lo, int hi, const T (&x)[kVecRows<T>]) {
+__device__ __forceinline__ void store_chunk(T* p, int cnt, bool aligned, const T (&x)[kVecRows<T>]) {
     constexpr int R = kVecRows<T>;
-    if (hi - lo == R) {
+    if (cnt == R && aligned) {
         if constexpr (R == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
         else *reinterpret_cast<double2*>(p) = make_double2(x[0], x[1]);
     } else {
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            if (r >= lo && r < hi) p[r] = x[r];
+            if (r < cnt) p[r] = x[r];
     }
 }
 
-// The tile of a multi-vector kernel seen by one thread: its first row (of the chunk) and the chunk's
-// rows inside the tile; group and place in the group follow from the thread index.
+// The tile [first, end) of a multi-vector kernel seen by one thread: its chunk's first row and rows;
+// group and place in the group follow from the thread index.
 template <typename T, class S>
 struct VecTile {
     static constexpr int kThreads = kBlk / S::kVS, kWarps = kThreads / 32;
     int32_t row0;
-    int lo, hi;
-    __device__ VecTile(int32_t first, int32_t beg, int32_t end) {
+    int cnt;
+    bool aligned;
+    __device__ VecTile(int32_t first, int32_t end, bool aligned_) : aligned(aligned_) {
         constexpr int R = kVecRows<T>;
         row0 = first + R * t();
-        lo = min(max(beg - row0, 0), R);
-        hi = max(min(end - row0, R), lo);
+        cnt = max(min(end - row0, R), 0);
     }
     static __device__ __forceinline__ int g() { return S::kVS == 1 ? 0 : (int)threadIdx.x / kThreads; }
     static __device__ __forceinline__ int t() { return S::kVS == 1 ? (int)threadIdx.x : (int)threadIdx.x % kThreads; }
 };
+
+// sum of the block's per-warp partials: two warps (64 chunks) at a time
+template <int NW>
+__device__ __forceinline__ double warps_sum(const double* red) {
+    double s = red[0] + red[1];
+#pragma unroll
+    for (int v = 2; v < NW; v += 2) s += red[v] + red[v + 1];
+    return s;
+}
 
 // red[i][warp of the group] = that warp's partial of <u_i, wt> for i < nvec (products in double)
 template <typename T, class S>
@@ -389,7 +438,7 @@ __device__ __forceinline__ void group_dots(const T* V, int64_t ldv, const VecTil
     for (int i = q.g(); i < nvec; i += GV * VS, p += GV * VS * ldv) {
         T x[GV][R];
 #pragma unroll
-        for (int u = 0; u < GV; ++u) load_chunk(p + u * VS * ldv, q.lo, i + u * VS < nvec ? q.hi : q.lo, x[u]);
+        for (int u = 0; u < GV; ++u) load_chunk(p + u * VS * ldv, i + u * VS < nvec ? q.cnt : 0, q.aligned, x[u]);
 #pragma unroll
         for (int u = 0; u < GV; ++u) {
             double sq = 0.0;
@@ -401,64 +450,117 @@ __device__ __forceinline__ void group_dots(const T* V, int64_t ldv, const VecTil
     }
 }
 
-// acc[r] = sum_i coef[i] u_i[row0 + r] for i < nvec: each group its vectors in order, then the groups
-// in order (s_acc: kBlk * R doubles, used when the block has several groups; one barrier then)
+// this block's partial of ||w||^2, valid in thread 0 (one barrier)
 template <typename T, class S>
-__device__ __forceinline__ void group_combine(const T* V, int64_t ldv, const VecTile<T, S>& q, const double* coef, int nvec, double* acc,
-                                              double* s_acc) {
-    constexpr int R = kVecRows<T>, GV = S::kGV, VS = S::kVS;
+__device__ __forceinline__ double tile_norm2(const VecTile<T, S>& q, const T* wt, double* red) {
+    if (q.g() == 0) {
+        double sq = 0.0;
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = 0.0;
-    const T* p = V + q.row0 + q.g() * ldv;
-    for (int i = q.g(); i < nvec; i += GV * VS, p += GV * VS * ldv) {
-        T x[GV][R];
-#pragma unroll
-        for (int u = 0; u < GV; ++u) load_chunk(p + u * VS * ldv, q.lo, i + u * VS < nvec ? q.hi : q.lo, x[u]);
-#pragma unroll
-        for (int u = 0; u < GV; ++u) {
-            if (i + u * VS < nvec) {
-                const double c = coef[i + u * VS];
-#pragma unroll
-                for (int r = 0; r < R; ++r) acc[r] += c * (double)x[u][r];
-            }
-        }
+        for (int r = 0; r < kVecRows<T>; ++r) sq += (double)wt[r] * (double)wt[r];
+        sq = warp_sum(sq);
+        if ((threadIdx.x & 31) == 0) red[q.t() >> 5] = sq;
     }
-    if constexpr (VS > 1) {
-        constexpr int TG = VecTile<T, S>::kThreads;
-#pragma unroll
-        for (int r = 0; r < R; ++r) s_acc[(q.g() * R + r) * TG + q.t()] = acc[r];
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            double a = s_acc[r * TG + q.t()];
-#pragma unroll
-            for (int g = 1; g < VS; ++g) a += s_acc[(g * R + r) * TG + q.t()];
-            acc[r] = a;
-        }
-    }
+    __syncthreads();
+    return threadIdx.x == 0 ? warps_sum<VecTile<T, S>::kWarps>(red) : 0.0;
 }
 
-// sums of the columns c0, c0 + step, ... < cnt of part[c][0..nb): a warp per column, four columns'
-// loads in flight; out(c, sum) is called by lane 0. For the few partials of a small system.
-template <typename F>
-__device__ __forceinline__ void sum_columns(const double* part, int64_t ld, int nb, int cnt, F out) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c0 = wid; c0 < cnt; c0 += 4 * nw) {
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int b = lane; b < nb; b += 32) {
+// w = win - sum_i coef[i] u_i (i < nvec) over the tile's rows; wt: the thread's chunk of w. The sum is one
+// of kChains chains (vectors c, c + kChains, ... in order), added in order: a block of several groups has
+// a chain per group, one of a single group takes them in turn. s_acc: kVecAcc doubles, one of the sums
+// per thread and row; out of registers, for the wide shape has none left.
+constexpr int kChains = 4;
+template <typename T, class S>
+constexpr int kVecAcc = kBlk * kVecRows<T>;
+
+template <typename T, class S>
+__device__ __forceinline__ void group_update(const T* V, int64_t ldv, const VecTile<T, S>& q, const double* coef, int nvec, const T* win, T* w,
+                                             double* s_acc, T (&wt)[kVecRows<T>]) {
+    constexpr int R = kVecRows<T>, GV = S::kGU, CA = sizeof(T) == 8 ? S::kCA : 1, VS = S::kVS, TG = VecTile<T, S>::kThreads;
+    static_assert(VS == 1 || VS == kChains, "a chain per group, or all of them in one");
+    double* mine = s_acc + q.g() * R * TG + q.t();
+#pragma unroll 1
+    for (int c = q.g(); c < kChains; c += VS * CA) {
+        double acc[CA][R];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (c0 + u * nw < cnt) s[u] += __ldcg(part + (int64_t)(c0 + u * nw) * ld + b);
+        for (int a = 0; a < CA; ++a)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[a][r] = 0.0;
+        const T* p = V + q.row0 + c * ldv;
+        for (int i = c; i < nvec; i += GV * kChains, p += GV * kChains * ldv) {
+            T x[GV][CA][R];
+#pragma unroll
+            for (int u = 0; u < GV; ++u)
+#pragma unroll
+                for (int a = 0; a < CA; ++a)
+                    load_chunk(p + (u * kChains + a) * ldv, i + u * kChains + a < nvec ? q.cnt : 0, q.aligned, x[u][a]);
+#pragma unroll
+            for (int u = 0; u < GV; ++u)
+#pragma unroll
+                for (int a = 0; a < CA; ++a) {
+                    if (i + u * kChains + a < nvec) {
+                        const double cf = coef[i + u * kChains + a];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) acc[a][r] += cf * (double)x[u][a][r];
+                    }
+                }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] = warp_sum(s[u]);
-        if (lane == 0) {
+        for (int a = 0; a < CA; ++a)
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (c0 + u * nw < cnt) out(c0 + u * nw, s[u]);
+            for (int r = 0; r < R; ++r) mine[r * TG] = VS > 1 || c + a == 0 ? acc[a][r] : mine[r * TG] + acc[a][r];
+    }
+    load_chunk(win + q.row0, q.cnt, q.aligned, wt);
+    if constexpr (VS > 1) __syncthreads();  // and every group has read win before group 0 overwrites it (win may be w)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        double a = s_acc[r * TG + q.t()];
+#pragma unroll
+        for (int g = 1; g < VS; ++g) a += s_acc[(g * R + r) * TG + q.t()];
+        wt[r] = (T)((double)wt[r] - a);  // rows past the end: 0 - 0
+    }
+    if (q.g() == 0) store_chunk(w + q.row0, q.cnt, q.aligned, wt);
+}
+
+// Up to this many partials per vector the update kernels sum them themselves: two launches per
+// Arnoldi step less (8,000 rows: 3.57 against 3.65 ms per solve; 400 partials already cost more than
+// the launches they save, 130 against 118 ms at 131,072 rows).
+constexpr int kFoldMax = 128;
+
+// sums of the columns c < cnt of part[c][0..nb), nb <= kFoldMax, with the bits of sum_groups: a warp per
+// column, several columns' loads in flight; out(c, sum) is called by lane 0. Lanes read consecutive
+// partials (every block reads all of them: L2 requests are what this costs); with PER = 4, four lanes'
+// values make a group, and the order of the sums is that of sum_groups with group q in lane q.
+template <int PER, typename F>
+__device__ __forceinline__ void sum_columns(const double* part, int64_t ld, int nb, int cnt, F out) {
+    static_assert(PER == 1 || PER == 4, "groups of one or of four lanes");
+    constexpr unsigned full = 0xffffffffu;
+    constexpr int kCols = PER > 1 ? 4 : 2, kL = kFoldMax / 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int c0 = wid; c0 < cnt; c0 += kCols * nw) {
+        double v[kCols][kL];
+#pragma unroll
+        for (int u = 0; u < kCols; ++u)
+#pragma unroll
+            for (int k = 0; k < kL; ++k)
+                v[u][k] = c0 + u * nw < cnt && lane + 32 * k < nb ? __ldcg(part + (int64_t)(c0 + u * nw) * ld + lane + 32 * k) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kCols; ++u) {
+            if constexpr (PER == 4) {
+#pragma unroll
+                for (int k = 0; k < kL; ++k) {
+                    if (32 * k >= nb) continue;
+                    const double b = __shfl_down_sync(full, v[u][k], 1), c = __shfl_down_sync(full, v[u][k], 2), d = __shfl_down_sync(full, v[u][k], 3);
+                    v[u][k] = v[u][k] + b + c + d;  // in every fourth lane
+                }
+            }
+            double s = (v[u][0] + v[u][2]) + (v[u][1] + v[u][3]);
+#pragma unroll
+            for (int o = 16; o >= PER; o >>= 1) s += __shfl_xor_sync(full, s, o);
+            if (lane == 0 && c0 + u * nw < cnt) out(c0 + u * nw, s);
         }
     }
 }
+static_assert(kFoldMax == 128, "four partials a lane");
 
 // ---------------------------------------------------------------- multi-dot (first CGS pass)
 // Per-block partials of d_i = <u_i, w> for i < nvec (summed by k_dots_finish<true>, or by k_update<FOLD>). with_norm: also the partials of ||w||^2, as vector nvec (the first pass
@@ -471,9 +573,9 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_mdot(KrylovDev K, const
     if (K.st->done || (only_reorth && !K.st->reorth)) return;
     __shared__ double red[kMaxBasis][kBlk / 32];
     constexpr int R = kVecRows<T>, NW = VecTile<T, S>::kWarps;
-    const VecTile<T, S> q((int32_t)(blockIdx.x * vec_block_rows<T, S>()), 0, (int32_t)K.n);
+    const VecTile<T, S> q((int32_t)(blockIdx.x * vec_block_rows<T, S>()), (int32_t)K.n, true);
     T wt[R];
-    load_chunk(w + q.row0, q.lo, q.hi, wt);
+    load_chunk(w + q.row0, q.cnt, q.aligned, wt);
     group_dots<T, S>(V, K.ldv, q, wt, nvec, red);
     if (with_norm && q.g() == 0) {
         double sq = 0.0;
@@ -485,12 +587,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_mdot(KrylovDev K, const
     __syncthreads();
     const int nout = nvec + (with_norm ? 1 : 0);
     double* part = K.part + (only_reorth ? (int64_t)kMaxBasis * K.nblk : 0);
-    for (int i = threadIdx.x; i < nout; i += blockDim.x) {
-        double s = 0.0;
-#pragma unroll
-        for (int v = 0; v < NW; ++v) s += red[i][v];
-        part[(int64_t)i * K.nblk + blockIdx.x] = s;
-    }
+    for (int i = threadIdx.x; i < nout; i += blockDim.x) part[(int64_t)i * K.nblk + blockIdx.x] = warps_sum<NW>(red[i]);
 }
 
 // Cross-block sums of the multi-dot partials, one warp per basis vector spread over the GPU (a
@@ -498,7 +595,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_mdot(KrylovDev K, const
 // nvec x nblk partials). FIRST: hacc_i = d_i / beta_i; else hacc_i += d_i / beta_i; both set
 // coef_i = d_i / beta_i^2 for the update that follows.
 // with_norm: warp nvec sums the partials of ||w||^2 into wnorm2; only_reorth as in k_mdot.
-template <bool FIRST>
+template <class S, bool FIRST>
 __global__ void __launch_bounds__(256) k_dots_finish(KrylovDev K, int nvec, int with_norm, int only_reorth) {
     pdl_wait();
     pdl_launch_dependents();
@@ -506,23 +603,7 @@ __global__ void __launch_bounds__(256) k_dots_finish(KrylovDev K, int nvec, int 
     const int lane = threadIdx.x & 31;
     const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (c >= nvec + (with_norm ? 1 : 0)) return;
-    const double* p = K.part + (int64_t)((FIRST ? 0 : kMaxBasis) + c) * K.nblk;
-    constexpr int kB = 16;
-    double s = 0.0;
-    for (int q0 = 0; q0 < K.nblk; q0 += 32 * kB) {
-        double v[kB];
-#pragma unroll
-        for (int k = 0; k < kB; ++k) {
-            const int q = q0 + lane + 32 * k;
-            v[k] = q < K.nblk ? p[q] : 0.0;
-        }
-#pragma unroll
-        for (int h = kB / 2; h > 0; h >>= 1)
-#pragma unroll
-            for (int k = 0; k < h; ++k) v[k] += v[k + h];
-        s += v[0];
-    }
-    s = warp_sum(s);
+    const double s = sum_groups<S::kPer>(K.part + (int64_t)((FIRST ? 0 : kMaxBasis) + c) * K.nblk, K.nblk);
     if (lane == 0 && c == nvec) {
         K.wnorm2[0] = s;
         return;
@@ -605,11 +686,11 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_update(KrylovDev K, con
     constexpr int R = kVecRows<T>, NW = VecTile<T, S>::kWarps;
     __shared__ double red[FINAL ? 1 : kMaxBasis][kBlk / 32];
     __shared__ double s_coef[kMaxBasis];
-    __shared__ double s_acc[S::kVS > 1 ? kBlk * R : 1];
+    __shared__ double s_acc[kVecAcc<T, S>];
     __shared__ ColumnSmem s_col;
     double* h = s_col.h;
     if constexpr (FOLD) {
-        sum_columns(K.part + (second ? (int64_t)kMaxBasis * K.nblk : 0), K.nblk, K.nblk, nvec, [&](int c, double s) {
+        sum_columns<S::kPer>(K.part + (second ? (int64_t)kMaxBasis * K.nblk : 0), K.nblk, K.nblk, nvec, [&](int c, double s) {
             const double ib = K.inv_beta[c], hc = s * ib, cf = hc * ib;
             s_coef[c] = cf;
             h[c] = second ? K.hacc[c] + hc : hc;
@@ -630,43 +711,28 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_update(KrylovDev K, con
             s_col.sn[i] = K.sn[i];
         }
     __syncthreads();
-    const VecTile<T, S> q((int32_t)(blockIdx.x * vec_block_rows<T, S>()), 0, (int32_t)K.n);
-    double acc[R];
-    group_combine<T, S>(V, K.ldv, q, s_coef, nvec, acc, s_acc);
+    const VecTile<T, S> q((int32_t)(blockIdx.x * vec_block_rows<T, S>()), (int32_t)K.n, true);
     T wt[R];
-    load_chunk(win + q.row0, q.lo, q.hi, wt);
-#pragma unroll
-    for (int r = 0; r < R; ++r) wt[r] = (T)((double)wt[r] - acc[r]);  // rows past the end: 0 - 0
-    if (S::kVS > 1) __syncthreads();  // every group has read win before group 0 overwrites it (win may be w)
-    if (q.g() == 0) store_chunk(w + q.row0, q.lo, q.hi, wt);
+    group_update<T, S>(V, K.ldv, q, s_coef, nvec, win, w, s_acc, wt);  // win may be w
     if (!FINAL) {
         group_dots<T, S>(V, K.ldv, q, wt, nvec, red);
         __syncthreads();
         double* part = K.part + (int64_t)kMaxBasis * K.nblk;
-        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-            double s = 0.0;
-#pragma unroll
-            for (int v = 0; v < NW; ++v) s += red[i][v];
-            part[(int64_t)i * K.nblk + blockIdx.x] = s;  // summed by k_dots_finish<false> or the next update
-        }
+        // summed by k_dots_finish<false> or the next update
+        for (int i = threadIdx.x; i < nvec; i += blockDim.x) part[(int64_t)i * K.nblk + blockIdx.x] = warps_sum<NW>(red[i]);
     } else {
-        double s = 0.0;
-        if (q.g() == 0) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) s += (double)wt[r] * (double)wt[r];
-        }
-        s = block_sum(s, red[0]);
+        const double s = tile_norm2<T, S>(q, wt, red[0]);
         double* part = K.part + (int64_t)2 * kMaxBasis * K.nblk;
         if (threadIdx.x == 0) publish_partial(part + blockIdx.x, s);
         if (!last_block_arrive(K.counter + 3)) return;
-        const double tot = reduce_partials(part, gridDim.x, red[0]);
+        const double tot = reduce_partials<S::kPer>(part, gridDim.x, red[0]);
         // first pass of the reorthogonalise-if-needed scheme (Daniel, Gragg, Kaufman & Stewart
         // 1976): a second pass only when the projection removed more than half of ||w||^2
         __shared__ int s_again;
         double wn2 = 0.0;
         if (dgks) {
             __syncthreads();
-            wn2 = FOLD ? reduce_partials(K.part + (int64_t)nvec * K.nblk, K.nblk, red[0]) : K.wnorm2[0];
+            wn2 = FOLD ? reduce_partials<S::kPer>(K.part + (int64_t)nvec * K.nblk, K.nblk, red[0]) : K.wnorm2[0];
         }
         if (threadIdx.x == 0) {
             K.counter[3] = 0u;
@@ -700,18 +766,12 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_zupdate(KrylovDev K, T*
     if (K.st->done) return;
     constexpr int R = kVecRows<T>;
     __shared__ double s_c[kMaxBasis];
-    __shared__ double s_acc[S::kVS > 1 ? kBlk * R : 1];
+    __shared__ double s_acc[kVecAcc<T, S>];
     for (int i = threadIdx.x; i < nvec; i += blockDim.x) s_c[i] = K.coefz[i];
     __syncthreads();
-    const VecTile<T, S> q((int32_t)(blockIdx.x * vec_block_rows<T, S>()), 0, (int32_t)K.n);
-    double acc[R];
-    group_combine<T, S>(Z, K.ldv, q, s_c, nvec, acc, s_acc);
-    if (q.g() != 0) return;
-    T qt[R];
-    load_chunk(qv + q.row0, q.lo, q.hi, qt);
-#pragma unroll
-    for (int r = 0; r < R; ++r) qt[r] = (T)((double)qt[r] - acc[r]);
-    store_chunk(Z + (int64_t)(j + 1) * K.ldv + q.row0, q.lo, q.hi, qt);
+    const VecTile<T, S> q((int32_t)(blockIdx.x * vec_block_rows<T, S>()), (int32_t)K.n, true);
+    T zt[R];
+    group_update<T, S>(Z, K.ldv, q, s_c, nvec, qv, Z + (int64_t)(j + 1) * K.ldv, s_acc, zt);
 }
 
 // ---------------------------------------------------------------- end of cycle

@@ -8,10 +8,12 @@
 // `done` flag. A mesh that has converged (or finished its m steps of the cycle) is masked out of the
 // orthogonalisation kernels; the cycle ends once every mesh is done.
 //
-// A mesh's iterates do not depend on the rest of the batch: the vector kernels work on tiles that lie
-// inside one mesh (the single-system kernels' tiles; the first one of a mesh that starts off a
-// 16-byte boundary is shorter by the offset, so that all others are aligned), the residual on tiles
-// of kBlk / kSpG rows, and every per-mesh sum runs over the mesh's own tiles in a fixed order.
+// A mesh's iterates have the bits of the same mesh solved alone: the vector kernels work on tiles that
+// start at the mesh's first row (the single-system kernels' tiles), the residual on tiles of kBlk / kSpG
+// rows, every per-mesh sum runs over the mesh's own tiles, and the orders of all sums are the same for
+// every shape of the vector kernels (which goes by the rows of the whole batch) and for folded sums
+// (which go by its largest mesh), as they are for both row layouts of the SpMV. A mesh that starts off a
+// 16-byte boundary moves its vectors row by row instead of in 16-byte chunks.
 #pragma once
 #include "krylov.cuh"
 
@@ -195,11 +197,11 @@ __global__ void __launch_bounds__(kBlk) k_bresid_finish(BatchDev B, int first, d
     batch_arrive(B, M->done != 0, conv);
 }
 
-// The tile of block t: chunks on 16-byte boundaries, rows outside the tile masked.
+// The tile of block t: a multiple of whole chunks behind its mesh's first row.
 template <typename T, class S>
 __device__ __forceinline__ VecTile<T, S> batch_tile(const BatchDev& B, int t) {
     const int32_t beg = (int32_t)B.tile_row[t];
-    return VecTile<T, S>(beg & ~(kVecRows<T> - 1), beg, (int32_t)B.tile_row[t + 1]);
+    return VecTile<T, S>(beg, (int32_t)B.tile_row[t + 1], (beg & (kVecRows<T> - 1)) == 0);
 }
 
 // First CGS pass: per-tile partial dots of the mesh's basis with w (k_mdot per tile).
@@ -214,19 +216,14 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bmdot(BatchDev B, const
     constexpr int R = kVecRows<T>, NW = VecTile<T, S>::kWarps;
     const VecTile<T, S> q = batch_tile<T, S>(B, t);
     T wt[R];
-    load_chunk(w + q.row0, q.lo, q.hi, wt);
+    load_chunk(w + q.row0, q.cnt, q.aligned, wt);
     group_dots<T, S>(V, B.ldv, q, wt, nvec, red);
     __syncthreads();
-    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-        double s = 0.0;
-#pragma unroll
-        for (int v = 0; v < NW; ++v) s += red[i][v];
-        B.part[(int64_t)i * B.ntile + t] = s;
-    }
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) B.part[(int64_t)i * B.ntile + t] = warps_sum<NW>(red[i]);
 }
 
 // Per-mesh cross-tile sums (k_dots_finish over the mesh's tiles): one warp per (mesh, vector).
-template <bool FIRST>
+template <class S, bool FIRST>
 __global__ void __launch_bounds__(256) k_bdots_finish(BatchDev B, int nvec) {
     pdl_wait();
     pdl_launch_dependents();
@@ -237,23 +234,7 @@ __global__ void __launch_bounds__(256) k_bdots_finish(BatchDev B, int nvec) {
     const int m = (int)(wgl / nvec), c = (int)(wgl % nvec);
     if (B.ms[m].done) return;
     const int t0 = B.mesh_tile[m], nt = B.mesh_tile[m + 1] - t0;
-    const double* p = B.part + (int64_t)((FIRST ? 0 : kMaxBasis) + c) * B.ntile + t0;
-    constexpr int kB = 16;
-    double s = 0.0;
-    for (int q0 = 0; q0 < nt; q0 += 32 * kB) {
-        double v[kB];
-#pragma unroll
-        for (int k = 0; k < kB; ++k) {
-            const int q = q0 + lane + 32 * k;
-            v[k] = q < nt ? p[q] : 0.0;
-        }
-#pragma unroll
-        for (int h = kB / 2; h > 0; h >>= 1)
-#pragma unroll
-            for (int k = 0; k < h; ++k) v[k] += v[k + h];
-        s += v[0];
-    }
-    s = warp_sum(s);
+    const double s = sum_groups<S::kPer>(B.part + (int64_t)((FIRST ? 0 : kMaxBasis) + c) * B.ntile + t0, nt);
     if (lane == 0) {
         const double ib = B.inv_beta[(int64_t)m * (B.m + 1) + c];
         double* hacc = B.hacc + (int64_t)m * kMaxBasis;
@@ -279,7 +260,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, con
     constexpr int R = kVecRows<T>, NW = VecTile<T, S>::kWarps;
     __shared__ double red[FINAL ? 1 : kMaxBasis][kBlk / 32];
     __shared__ double s_coef[kMaxBasis];
-    __shared__ double s_acc[S::kVS > 1 ? kBlk * R : 1];
+    __shared__ double s_acc[kVecAcc<T, S>];
     __shared__ ColumnSmem s_col;
     const int m1 = B.m + 1;
     const int t0 = B.mesh_tile[m], nt = B.mesh_tile[m + 1] - t0;
@@ -288,7 +269,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, con
     double* sn = B.sn + (int64_t)m * B.m;
     const double* inv_beta = B.inv_beta + (int64_t)m * m1;
     if constexpr (FOLD) {
-        sum_columns(B.part + (FINAL ? (int64_t)kMaxBasis * B.ntile : 0) + t0, B.ntile, nt, nvec, [&](int c, double s) {
+        sum_columns<S::kPer>(B.part + (FINAL ? (int64_t)kMaxBasis * B.ntile : 0) + t0, B.ntile, nt, nvec, [&](int c, double s) {
             const double ib = inv_beta[c], hc = s * ib;
             s_coef[c] = hc * ib;
             s_col.h[c] = FINAL ? hacc[c] + hc : hc;
@@ -307,31 +288,15 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, con
         }
     __syncthreads();
     const VecTile<T, S> q = batch_tile<T, S>(B, t);
-    double acc[R];
-    group_combine<T, S>(V, B.ldv, q, s_coef, nvec, acc, s_acc);
     T wt[R];
-    load_chunk(win + q.row0, q.lo, q.hi, wt);
-#pragma unroll
-    for (int r = 0; r < R; ++r) wt[r] = (T)((double)wt[r] - acc[r]);  // rows outside the tile: 0 - 0
-    if (S::kVS > 1) __syncthreads();  // every group has read win before group 0 overwrites it (win may be w)
-    if (q.g() == 0) store_chunk(w + q.row0, q.lo, q.hi, wt);
+    group_update<T, S>(V, B.ldv, q, s_coef, nvec, win, w, s_acc, wt);  // win may be w
     if (!FINAL) {
         group_dots<T, S>(V, B.ldv, q, wt, nvec, red);
         __syncthreads();
         double* part = B.part + (int64_t)kMaxBasis * B.ntile;
-        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-            double s = 0.0;
-#pragma unroll
-            for (int v = 0; v < NW; ++v) s += red[i][v];
-            part[(int64_t)i * B.ntile + t] = s;
-        }
+        for (int i = threadIdx.x; i < nvec; i += blockDim.x) part[(int64_t)i * B.ntile + t] = warps_sum<NW>(red[i]);
     } else {
-        double s = 0.0;
-        if (q.g() == 0) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) s += (double)wt[r] * (double)wt[r];
-        }
-        s = block_sum(s, red[0]);
+        const double s = tile_norm2<T, S>(q, wt, red[0]);
         double* part = B.part + (int64_t)2 * kMaxBasis * B.ntile;
         __shared__ bool s_last;
         if (threadIdx.x == 0) {
@@ -341,7 +306,7 @@ __global__ void __launch_bounds__(kBlk, S::kMinBlocks) k_bupdate(BatchDev B, con
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        const double tot = reduce_partials(part + t0, nt, red[0]);
+        const double tot = reduce_partials<S::kPer>(part + t0, nt, red[0]);
         double* g = B.g + (int64_t)m * m1;
         const ColumnDst D{B.H + ((int64_t)m * B.m + j) * m1, cs, sn, g, B.beta + (int64_t)m * m1, B.inv_beta + (int64_t)m * m1};
         const ColumnEnd c = arnoldi_column(D, s_col, j, tot);
