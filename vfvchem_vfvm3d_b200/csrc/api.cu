@@ -993,14 +993,15 @@ struct Gmres : SolverBase {
     DBuf<DevStatus> st;
     KrylovDev K{};
     // Cycle graphs by the number of leading steps that run unconditionally (CycleGraph), the steps that
-    // each cycle of the last solve took, and how often a graph was wanted that is not built
+    // each cycle of the last solve and of the one before took, and how often a graph was wanted that is
+    // not built
     struct CycleGraph {
         cudaGraphExec_t exec = nullptr;
         int64_t nodes = 0, step_nodes = 0;  // kernels of the unconditional part, of one conditional step
     };
     std::map<int, CycleGraph> graphs;
     std::map<int, int> wanted;
-    std::vector<int> last_cycles;
+    std::vector<int> last_cycles, older_cycles;
     IluStruct* ilu = nullptr;
     uint64_t bj_version = ~0ull, valk_version = ~0ull;  // versions of the pattern's values behind binv and valK
     // overlapped engine: preconditioned basis Z, SpMV output a, q = M^-1 a, the second stream
@@ -1666,15 +1667,21 @@ struct Gmres : SolverBase {
 
     // The graph of the next cycle. An IF node costs ~12 us whether its steps run or not (3 us per
     // Arnoldi step: 3.70 against 3.23 ms for 150 steps on 8,000 rows with none), so the steps that a
-    // cycle is expected to take anyway - as many as the same cycle of the last solve took, or all m
-    // after a full cycle - run unconditionally. Which graph runs never changes a result: a step after
-    // convergence does nothing. A graph takes milliseconds to build, so one is added only when it has
+    // cycle is expected to take anyway - as many as the same cycle of the last solve took, and of the one
+    // before (a program that goes to and fro between long and short solves on one handle would run the
+    // long one's steps, ~25 kernels each that do nothing, in every short one), or all m after a full
+    // cycle - run unconditionally. Which graph runs never changes a result: a step after convergence does
+    // nothing. A graph takes milliseconds to build, so one is added only when it has
     // been wanted kWantedOften times, at most kMaxGraphs per solver; otherwise the one with the most
     // leading steps up to the expected number is taken.
     void pick_graph(vfv_ctx* ctx, vfv_pattern* p, int cycle, const std::vector<int>& took, const CycleGraph** out, int* lead) {
         int want = 0;
-        if (cycle < (int)last_cycles.size()) want = last_cycles[cycle];
-        else if (!took.empty() && took.back() >= m) want = m;
+        if (cycle < (int)last_cycles.size()) {
+            want = last_cycles[cycle];
+            if (!older_cycles.empty()) want = std::min(want, cycle < (int)older_cycles.size() ? older_cycles[cycle] : 0);
+        } else if (!took.empty() && took.back() >= m) {
+            want = m;
+        }
         want = std::max(0, std::min(want, m));
         if (graphs.begin()->first == 0 && want > 0 && !graphs.count(want) && (int)graphs.size() < kMaxGraphs && ++wanted[want] == kWantedOften)
             add_graph(ctx, p, want);  // where it cannot be built the others serve
@@ -1829,6 +1836,7 @@ struct Gmres : SolverBase {
             }
             ++cycles;
         }
+        older_cycles.swap(last_cycles);
         last_cycles.swap(took);
         CK(cudaGetLastError());
         if (trace.p) dump_trace(ctx, cycles);
