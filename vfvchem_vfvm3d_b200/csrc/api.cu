@@ -1646,8 +1646,9 @@ struct Gmres : SolverBase {
         return cudaSuccess;
     }
 
-    // captures, instantiates and keeps the cycle graph with `lead` unconditional steps
-    int add_graph(vfv_ctx* ctx, vfv_pattern* p, int lead) {
+    // captures, instantiates and keeps the cycle graph with `lead` unconditional steps; sets no error text,
+    // for a solve goes on without a graph that cannot be built while it has another
+    cudaError_t add_graph(vfv_ctx* ctx, vfv_pattern* p, int lead) {
         cudaGraph_t graph = nullptr;
         CycleGraph g;
         cudaError_t e = build_cycle_graph(ctx->stream, p, lead, &graph, &g.nodes, &g.step_nodes);
@@ -1659,10 +1660,10 @@ struct Gmres : SolverBase {
             if (const char* t = getenv("VFV_TRACE_SOLVE"))
                 if (t[0] == '1') fprintf(stderr, "[vfv] cycle graph with %d leading steps not built: %s\n", lead, cudaGetErrorString(e));
             cudaGetLastError();
-            return set_err(ctx, VFV_CUDA_ERROR, std::string("cycle graph: ") + cudaGetErrorString(e));
+            return e;
         }
         graphs.emplace(lead, g);
-        return VFV_OK;
+        return cudaSuccess;
     }
 
     // The graph of the next cycle. An IF node costs ~12 us whether its steps run or not (3 us per
@@ -1784,9 +1785,9 @@ struct Gmres : SolverBase {
         }
         if (engine != VFV_ENGINE_PERSISTENT && graphs.empty()) {
             // conditional steps unless asked for the straight graph or refused by the driver
-            int rc = getenv("VFV_STRAIGHT_GRAPH") ? VFV_CUDA_ERROR : add_graph(ctx, p, 0);
-            if (rc) rc = add_graph(ctx, p, m);
-            if (rc) return rc;
+            cudaError_t e = getenv("VFV_STRAIGHT_GRAPH") ? cudaErrorNotSupported : add_graph(ctx, p, 0);
+            if (e != cudaSuccess) e = add_graph(ctx, p, m);
+            if (e != cudaSuccess) return set_err(ctx, VFV_CUDA_ERROR, std::string("cycle graph: ") + cudaGetErrorString(e));
         }
         int cycles = 0, rc = VFV_OK, steps_seen = 0;
         std::vector<int> took;            // steps of this solve's cycles
