@@ -960,8 +960,15 @@ int build_pattern_sell(vfv_ctx* ctx, vfv_pattern* p) {
 #pragma omp parallel for schedule(static)
     for (int64_t r = 0; r < p->n; ++r)
         for (int32_t q = 0; q < p->h_rp[r + 1] - p->h_rp[r]; ++q) ci[h.slot(r, q)] = p->h_ci[p->h_rp[r] + q];
-    CK(p->sell.upload(h, ctx->stream));
-    CK(p->sell_ci.upload(ci.data(), ci.size(), ctx->stream));
+    cudaError_t e = p->sell.upload(h, ctx->stream);
+    if (e == cudaSuccess) e = p->sell_ci.upload(ci.data(), ci.size(), ctx->stream);
+    if (e == cudaErrorMemoryAllocation) {  // another process was faster: the CSR rows are there
+        cudaGetLastError();
+        p->sell.release();
+        p->sell_ci.release();
+        return VFV_OK;
+    }
+    CK(e);
     p->sell_use = true;
     return VFV_OK;
 }
@@ -1126,7 +1133,16 @@ struct Gmres : SolverBase {
         }
         sell = may_sell && p->sell_use;
         if (sell) {
-            CK(valK.alloc(std::max<int64_t>(p->sell.slots, 1)));
+            const cudaError_t e = valK.alloc(std::max<int64_t>(p->sell.slots, 1));
+            if (e == cudaErrorMemoryAllocation) {  // no room beside the CSR rows: solve from those
+                cudaGetLastError();
+                valK.release();
+                sell = false;
+            } else {
+                CK(e);
+            }
+        }
+        if (sell) {
             CK(cudaMemsetAsync(valK.p, 0, valK.n * sizeof(T), ctx->stream));  // padding
         } else if (need_copy) {
             CK(valK.alloc(p->nnz));

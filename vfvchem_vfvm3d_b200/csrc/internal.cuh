@@ -138,6 +138,12 @@ struct SellBuf {
         if (e == cudaSuccess) e = tail.upload(h.tail.data(), h.tail.size(), s);
         return e;
     }
+    void release() {
+        so.release();
+        tail.release();
+        p8.release();
+        r8.release();
+    }
     SellDev dev() const { return {so.p, p8.p, r8.p, tail.p}; }
 };
 
