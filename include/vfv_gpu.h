@@ -270,7 +270,8 @@ int vfv_update_grad(vfv_ctx* ctx, vfv_heat* h, const double* f, double* grad);
  * Per row, in push order: OpSclDomTimeUnity (opscl_dom_timeunity.rs:32-58), OpSclDomDiffusion
  * (opscl_dom_diff.rs:40-91), OpSclDomAdvection (power law, opscl_dom_adv.rs:49-125) with the face mass
  * flux of flow_helper::update_flux (flow_helper.rs:72-179) at zero pressure and body force; density
- * and species weight 1. The reference has no solver that wires this composition (TransientMass has
+ * and species weight 1; the diagonal's sums over a row's faces are split over lanes, in a fixed order.
+ * The reference has no solver that wires this composition (TransientMass has
  * no advection). */
 int vfv_transport_create(vfv_ctx* ctx, int nmesh, vfv_mesh* const* meshes, double dt, vfv_transport** out);
 void vfv_transport_destroy(vfv_transport* t);

@@ -78,7 +78,6 @@ void SellHost::build(int64_t n_, const int32_t* rp) {
         tot += 32 * (int64_t)w[sl];
         so[sl + 1] = (int32_t)tot;
     }
-    first_tail = tot;
     tail.clear();
     if (tails > 0) {
         tail.resize(n + 1);
@@ -934,8 +933,9 @@ VecShape vec_shape(int64_t rows) {
 }
 
 // The sliced rows of a pattern's SpMV: wanted
-//  - for a full wave of the sliced kernel's resident blocks, 148 x 5 x 256 rows: with fewer, a thread
-//    per row leaves the chip idle and several lanes per CSR row are faster (8,000 rows: 3.27 against
+//  - for 148 SMs x 5 blocks x 256 rows, what a B200 keeps resident of the double kernel (the float ones
+//    have six to eight blocks an SM; one line for both, as 103,823 rows show nothing to gain): with fewer,
+//    a thread per row leaves the chip idle and several lanes per CSR row are faster (8,000 rows: 3.27 against
 //    3.56 ms per solve; 103,823: 10.1 / 10.4; 125,000 double: 40.9 / 42.4; 262,144 double: 32.8 / 32.4;
 //    10^6 float: 93.0 / 87.7);
 //  - where every row is short and like its neighbours (no tails, no slice wider than kSellMost): a

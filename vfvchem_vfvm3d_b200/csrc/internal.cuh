@@ -101,7 +101,7 @@ inline int grid_for(int64_t threads, int block = 256) { return (int)std::max<int
 constexpr int kSellWindow = 256;
 
 struct SellHost {
-    int64_t n = 0, slots = 0, first_tail = 0;
+    int64_t n = 0, slots = 0;
     std::vector<int32_t> so;    // [positions / 32 + 1] first slot of each slice
     std::vector<uint8_t> p8;    // [positions] offset in the window of the row at this position
     std::vector<uint8_t> r8;    // [positions] position in the window of this row

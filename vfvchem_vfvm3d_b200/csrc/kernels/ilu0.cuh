@@ -310,8 +310,9 @@ __global__ void __launch_bounds__(32 * kFacWarps) k_ilu0_factor_level_warp(int32
 // levels: the lower entries are sorted by level) are eliminated while the last ones are waited for.
 // Flags and fences -> values: 103,823 rows (319 levels) 1.37 -> 0.71 ms, 10^6 rows (692 levels)
 // 4.10 -> 2.77 ms: 2.2 us a level where few rows are in flight; at 10^6 the rows' own work (10 us for
-// the structure, the polls and the eliminations of a row, on 3,552 warps) bounds it. Four blocks per
-// SM (64 registers, spills) take 3.4 ms, two (125 registers, no prefetch) 4.05. k_ilu0_factor_flags (ready[k] == epoch once row k is
+// the structure, the polls and the eliminations of a row, on 3,552 warps) bounds it. Three blocks
+// per SM (80 registers, 28 bytes of them spilled); four (64, more spills) take 3.4 ms, two (125, no
+// prefetch) 4.05. k_ilu0_factor_flags (ready[k] == epoch once row k is
 // final) takes patterns with rows beyond the staging, whose serial rows work in place.
 __global__ void __launch_bounds__(32 * kFacWarps) k_ilu0_factor_flags(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                                                       const int32_t* __restrict__ dg, double* a, int* __restrict__ bad,

@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(256) k_ns_mom_rows(NsDev D) {
 // 110,592 vertices on one B200: 0.99 ms cold, against 1.94 ms to write the triplets and 4.25 ms to sum
 // them per slot (630 M triplets through HBM twice). It is bound by the latency of L2 (one to two
 // instructions per scheduler every three cycles at 24 warps per SM): loading a face ahead took it from
-// 1.47 ms, 80 registers (6 blocks) against 96 (5) and 128 (4) 1.70, 1.75 and 1.87 ms per assembly.
+// 1.47 ms, 80 registers (6 blocks; 164 to 208 bytes spilled) against 96 (5) and 128 (4) 1.70, 1.75 and 1.87 ms per
+// assembly.
 constexpr int kPWarps = 4;
 constexpr int kPFaces = 32;  // faces staged at a time
 constexpr int kPU = 3;       // grad_coeff entries of a neighbour per lane in flight
